@@ -98,8 +98,8 @@ struct NsrArgs
     float referencePower;
     int resetInterval;
 };
-// Moving-mean-square buffer (srcStride floats per sample), per-reset-block maxima and the prefix.
-size_t nsr_scratch_bytes(int n, uint32_t srcStride, int resetInterval);
+// Prefix energies of the samples' 64-sample chunks (FP64).
+size_t nsr_scratch_bytes(int n, uint32_t srcStride);
 void launch_nsr(Handle& h, void* scratch, const NsrArgs& a);
 
 // Mel filter placement parameters (maxFreq already resolved: 0 -> sampleRate / 2).

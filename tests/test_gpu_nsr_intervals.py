@@ -1,0 +1,60 @@
+"""non_silent_region_detection decides from energy intervals and replays a reset block's float chain only where
+they do not settle an end: inputs at the edges of that rule, whole numbers equal to the oracle's."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from gpu_util import dev, host  # noqa: E402
+from rpp_b200 import audio  # noqa: E402
+from rpp_b200.types import audio_desc  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+
+def clips(seed):
+    """One clip per situation, of 3 samples to 41000, zero-padded into one batch."""
+    r = np.random.default_rng(seed)
+    noise = lambda n, a=0.3: r.normal(0, a, n).astype(np.float32)  # noqa: E731
+    quiet_end = noise(30000)
+    quiet_end[21000:] = 0.0                                  # the running sum decays to rounding residue
+    quiet_begin = noise(30000)
+    quiet_begin[:9000] = 0.0                                 # a whole silent reset block of 8192
+    island = np.zeros(41000, np.float32)
+    island[20000:20100] = noise(100)
+    floor = noise(40000, 1e-3)                               # a floor 60 dB below the loud part, give or take
+    floor[15000:25000] = noise(10000, 1.0)
+    fade = (noise(40000) * np.exp(-np.arange(40000) / 2500.0)).astype(np.float32)
+    gaps = noise(33000)
+    for s in range(0, 33000, 6000):
+        gaps[s:s + 3500] = 0.0
+    flat = np.full(20000, 0.1, np.float32)                   # every full window ties with the maximum
+    spike = np.zeros(10000, np.float32)
+    spike[[0, 9999]] = 0.5, 0.7
+    big = noise(9000)
+    big[4000] = np.inf
+    return [quiet_end, quiet_begin, island, floor, fade, gaps, flat, spike, big, noise(12000, 1e-21),
+            np.zeros(5000, np.float32), noise(3), noise(63), noise(64), noise(65), noise(8192), noise(8193),
+            noise(2048, 1e-6), np.zeros(0, np.float32), np.concatenate([noise(8192, 1e-4), noise(8192, 1.0), noise(9000, 1e-4)])]
+
+
+@pytest.mark.parametrize("pad", [0, 3])
+@pytest.mark.parametrize("reset,window,ref,cut", [
+    (8192, 2048, 0.0, -60.0), (8192, 2048, 0.0, 0.0), (8192, 2048, 0.0, -0.05), (8192, 2048, 0.0, -120.0),
+    (4096, 256, 0.0, -40.0), (4096, 255, 0.0, -40.0), (1000, 333, 0.0, -59.9), (64, 512, 0.0, -30.0),
+    (63, 512, 0.0, -30.0), (-1, 2048, 0.0, -60.0), (100, 4096, 0.0, -80.0), (8192, 65536, 0.0, -20.0),
+    (8192, 2048, 0.09, 0.0), (8192, 2048, 0.01, 0.0), (8192, 2048, -1.0, -20.0), (8192, 2048, 1e-30, -30.0)])
+def test_region_equals_oracle(gpu, oracle, reset, window, ref, cut, pad):
+    c = clips(5)
+    lens = np.array([len(v) for v in c], np.int32)
+    x = np.zeros((len(c), int(lens.max()) + pad), np.float32)   # pad 3: rows that are not 16-byte aligned
+    for i, v in enumerate(c):
+        x[i, :len(v)] = v
+    with np.errstate(over="ignore", invalid="ignore"):
+        b_ref, l_ref = oracle.nsr(x, lens, cut, window, ref, reset)
+    begin = torch.full((len(lens),), -7, dtype=torch.int32, device="cuda")
+    length = torch.full((len(lens),), -7, dtype=torch.int32, device="cuda")
+    assert audio.non_silent_region_detection(dev(x), audio_desc(len(lens), x.shape[1]), dev(lens), begin, length, cut,
+                                             window, ref, reset, gpu) == 0
+    np.testing.assert_array_equal(host(begin), b_ref)
+    np.testing.assert_array_equal(host(length), l_ref)
