@@ -134,6 +134,16 @@ inline void launch_ragged_prefix(Count count, int n, long long* prefix, cudaStre
 // completed and its writes are visible (a no-op for a kernel launched the ordinary way).
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// The pointer to something that the kernel waited for has written, to be taken after grid_dependency_wait():
+// through a const __restrict__ parameter the compiler may load before the wait (it takes the memory for
+// constant), through the returned pointer it cannot.
+template <class T>
+__device__ __forceinline__ T* dependency_result(T* p)
+{
+    asm volatile("" : "+l"(p)::"memory");
+    return p;
+}
+
 // Launches `kernel` with programmatic stream serialization: it may start while the kernel before
 // it (which must allow it, as ragged_prefix_kernel does) is still running, so its setup overlaps
 // that kernel and the launch gap; it must call grid_dependency_wait() before touching that

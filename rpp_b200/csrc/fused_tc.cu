@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(kFusedThreads, 2)
     const int nslots = a.n + a.lookahead;
     __shared__ long long s_prefix[kFusedPrefixCache];
     grid_dependency_wait();   // the prefix and the zeroed counters of the prefix kernel
-    prefix = cache_prefix<kFusedPrefixCache>(prefix, nslots, s_prefix);
+    prefix = cache_prefix<kFusedPrefixCache>(dependency_result(prefix), nslots, s_prefix);
     const long long total = prefix[nslots];
     const SlotCount<TF> cnt{a, a.n, a.lookahead};
     const int fcol = 2 * (threadIdx.x % (TF / 2));   // first of the two frame columns this thread owns in mel tiles

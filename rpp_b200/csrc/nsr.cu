@@ -547,7 +547,7 @@ __global__ void __launch_bounds__(kThreads) region_kernel(const float* __restric
         }
         return;
     }
-    double* P = energies + b * pitch;
+    double* P = dependency_result(energies) + b * pitch;
     double* held = reinterpret_cast<double*>(buf);
     Clip clip{src + size_t(b) * stride, L, windowLength, reset == -1 ? L : reset,
               __fdiv_rn(1.0f, float(windowLength)), P, P, (L + kSub - 1) / kSub, 0.0, 0.0};
