@@ -52,6 +52,14 @@ __device__ bool check_range(const void* p, unsigned long long bytes, bool write,
 #define RPPB_RANGE_OK(p, bytes) true
 #endif
 
+// A function kept out of line so that its registers do not come on top of its caller's.  Inlined in the checked
+// build: relocatable code gives a function of its own more registers than a capped kernel may call.
+#ifdef RPPB_CHECKED
+#define RPPB_OUT_OF_LINE __forceinline__
+#else
+#define RPPB_OUT_OF_LINE __noinline__
+#endif
+
 // ---------------------------------------------------------------- ragged batches
 // A batch of uneven samples is addressed as one flat list of work units (chunks, frame tiles,
 // reset blocks ...).  prefix[b] is the number of units of samples 0..b-1 (prefix[n] = total),

@@ -414,13 +414,13 @@ RppStatus resample_common(Handle& h, RppPtr_t srcPtr, RpptDescPtr srcDescPtr, Rp
     m.take<float>(n);
     m.take<int>(2 * n);
     m.take<float>(lutSize);
-    m.take<char>(prefix_bytes(n));
+    m.take<char>(resample_scratch_bytes(n));
     Carver cv(h.workspace(m.used()));
     float* inStage = cv.take<float>(n);
     float* outStage = cv.take<float>(n);
     int* dimsStage = cv.take<int>(2 * n);
     float* lutStage = cv.take<float>(lutSize);
-    void* scratch = cv.take<char>(prefix_bytes(n));
+    void* scratch = cv.take<char>(resample_scratch_bytes(n));
     ResampleWindowDev win;
     win.lut = static_cast<const float*>(h.device_view(lutHost, lutSize * sizeof(float), lutStage));
     win.lutSize = lutSize;
@@ -433,7 +433,7 @@ RppStatus resample_common(Handle& h, RppPtr_t srcPtr, RpptDescPtr srcDescPtr, Rp
                     static_cast<const float*>(h.device_view(inRateTensor, n * sizeof(float), inStage)),
                     static_cast<const float*>(h.device_view(outRateTensor, n * sizeof(float), outStage)),
                     static_cast<const int*>(h.device_view(srcDimsTensor, 2 * n * sizeof(int), dimsStage)), win,
-                    downmix, normalize);
+                    int(srcDescPtr->c), downmix, normalize);
     return RPP_SUCCESS;
 }
 

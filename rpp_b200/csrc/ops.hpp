@@ -28,11 +28,14 @@ struct ResampleWindowDev
     // take the exact walk (every tap position exact in float; resample.cu)
     int exactMinE = 1 << 30, exactMaxE = -(1 << 30);
 };
+// The work-list prefix and the item counter.
+size_t resample_scratch_bytes(int n);
 // downmix: the input is interleaved {length, channels} and is down-mixed to mono while resampling
-// (equal to rppt_down_mixing_gpu followed by a mono rppt_resample_gpu).
+// (equal to rppt_down_mixing_gpu followed by a mono rppt_resample_gpu).  channels: the source descriptor's (it picks
+// the kernel; the samples' own counts are dims').
 void launch_resample(Handle& h, void* scratch, const float* src, uint32_t srcStride, float* dst, uint32_t dstStride, int n,
                      const float* inRate, const float* outRate, const int* dims, const ResampleWindowDev& win,
-                     bool downmix = false, bool normalize = false);
+                     int channels, bool downmix, bool normalize);
 // Mono resample of a clip table: clips[b].src (length at inRate) -> clips[b].work at outRate.
 void launch_resample_clips(Handle& h, void* scratch, const RppbClip* clips, int n, float outRate,
                            const ResampleWindowDev& win);

@@ -214,6 +214,79 @@ __device__ __forceinline__ float2 pair_at(uint32_t a)
     return v;
 }
 
+// One output of a mono signal with the reference's operations: 4 lanes, folded as (l0 + l2) + (l1 + l3),
+// then a scalar tail.
+template <class W, class At>
+__device__ __forceinline__ float mono_taps(const W& win, At at, int loc0, int loc1, float inPos)
+{
+    int l = loc0;
+    const float locBegin = __fsub_rn(float(l), inPos);
+    float lane4[4] = {__fadd_rn(locBegin, 0.f), __fadd_rn(locBegin, 1.f), __fadd_rn(locBegin, 2.f),
+                      __fadd_rn(locBegin, 3.f)};
+    float acc4[4] = {0.f, 0.f, 0.f, 0.f};
+    for (; l + 3 < loc1; l += 4)
+    {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+        {
+            acc4[q] = __fadd_rn(acc4[q], __fmul_rn(at(l + q), win.lane(lane4[q])));
+            lane4[q] = __fadd_rn(lane4[q], 4.f);
+        }
+    }
+    float accum = __fadd_rn(__fadd_rn(acc4[0], acc4[2]), __fadd_rn(acc4[1], acc4[3]));
+    float xx = __fsub_rn(float(l), inPos);
+    for (; l < loc1; ++l, xx = __fadd_rn(xx, 1.f)) accum = __fadd_rn(accum, __fmul_rn(at(l), win.scalar(xx)));
+    return accum;
+}
+
+// The same by the exact walk (resample_exact_range): the first tap's pair entry and weight by the same operations,
+// then each tap 32 entries (256 bytes) further on at that weight; the same products and sums in the same order.
+template <class W, class At>
+__device__ __forceinline__ float mono_taps_exact(const W& win, At at, int loc0, int loc1, float inPos)
+{
+    constexpr float kM = 12582912.0f;   // 1.5 * 2^23
+    const float locRaw = __fmaf_rn(__fsub_rn(float(loc0), inPos), win.scale, win.center);
+    const float m = __fadd_rd(locRaw, kM);
+    const float w = __fsub_rn(locRaw, __fsub_rn(m, kM));
+    uint32_t a = win.bias + (uint32_t(__float_as_int(m)) << 3);
+    auto tap = [&](int l, float2 e) { return __fmul_rn(at(l), __fadd_rn(e.x, __fmul_rn(w, e.y))); };
+    int l = loc0;
+    float acc4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 2
+    for (; l + 3 < loc1; l += 4, a += 4 * 256)
+    {
+        acc4[0] = __fadd_rn(acc4[0], tap(l, pair_at<0>(a)));
+        acc4[1] = __fadd_rn(acc4[1], tap(l + 1, pair_at<256>(a)));
+        acc4[2] = __fadd_rn(acc4[2], tap(l + 2, pair_at<512>(a)));
+        acc4[3] = __fadd_rn(acc4[3], tap(l + 3, pair_at<768>(a)));
+    }
+    float accum = __fadd_rn(__fadd_rn(acc4[0], acc4[2]), __fadd_rn(acc4[1], acc4[3]));
+    for (; l < loc1; ++l, a += 256) accum = __fadd_rn(accum, tap(l, pair_at<0>(a)));
+    return accum;
+}
+
+// One output of an interleaved multi-channel signal: per channel, in order.
+template <class W>
+__device__ __forceinline__ void channel_taps(const W& win, const float* in, float* out, int C, int loc0, int loc1,
+                                             float inPos)
+{
+    constexpr int kMaxC = 16;
+    float acc[kMaxC];
+#pragma unroll
+    for (int c = 0; c < kMaxC; ++c) acc[c] = 0.f;
+    float xx = __fsub_rn(float(loc0), inPos);
+    for (int l = loc0; l < loc1; ++l, xx = __fadd_rn(xx, 1.f))
+    {
+        const float wv = win.scalar(xx);
+#pragma unroll
+        for (int c = 0; c < kMaxC; ++c)
+            if (c < C) acc[c] = __fadd_rn(acc[c], __fmul_rn(__ldg(RPPB_RD(in + (long long)l * C + c)), wv));
+    }
+#pragma unroll
+    for (int c = 0; c < kMaxC; ++c)
+        if (c < C) *RPPB_WR(out + c) = acc[c];
+}
+
 // A unit of the flat work list, decoded by the phase warp for the compute warps.
 constexpr int kUnitSkip = 0, kUnitCopy = 1, kUnitResample = 2;
 struct UnitInfo
@@ -411,55 +484,8 @@ __global__ void __launch_bounds__(kThreads, 4)
                             if (loc1 + inBlockRounded > L) loc1 = L - inBlockRounded;
                             if (kMix || C == 1)
                             {
-                                // mono input: 4 lanes, folded as (l0 + l2) + (l1 + l3), then a scalar tail
-                                auto taps = [&](auto at) {
-                                    int l = loc0;
-                                    const float locBegin = __fsub_rn(float(l), inPos);
-                                    float lane4[4] = {__fadd_rn(locBegin, 0.f), __fadd_rn(locBegin, 1.f),
-                                                      __fadd_rn(locBegin, 2.f), __fadd_rn(locBegin, 3.f)};
-                                    float acc4[4] = {0.f, 0.f, 0.f, 0.f};
-                                    for (; l + 3 < loc1; l += 4)
-                                    {
-#pragma unroll
-                                        for (int q = 0; q < 4; ++q)
-                                        {
-                                            acc4[q] = __fadd_rn(acc4[q], __fmul_rn(at(l + q), win.lane(lane4[q])));
-                                            lane4[q] = __fadd_rn(lane4[q], 4.f);
-                                        }
-                                    }
-                                    float accum = __fadd_rn(__fadd_rn(acc4[0], acc4[2]), __fadd_rn(acc4[1], acc4[3]));
-                                    float xx = __fsub_rn(float(l), inPos);
-                                    for (; l < loc1; ++l, xx = __fadd_rn(xx, 1.f))
-                                        accum = __fadd_rn(accum, __fmul_rn(at(l), win.scalar(xx)));
-                                    return accum;
-                                };
-                                // the exact walk: the first tap's pair entry and weight by the same operations
-                                // as above, then each tap 32 entries (256 bytes) further on at that weight; the
-                                // same products and sums in the same order
-                                auto taps_exact = [&](auto at) {
-                                    constexpr float kM = 12582912.0f;   // 1.5 * 2^23
-                                    const float locRaw =
-                                        __fmaf_rn(__fsub_rn(float(loc0), inPos), win.scale, win.center);
-                                    const float m = __fadd_rd(locRaw, kM);
-                                    const float w = __fsub_rn(locRaw, __fsub_rn(m, kM));
-                                    uint32_t a = win.bias + (uint32_t(__float_as_int(m)) << 3);
-                                    auto tap = [&](int l, float2 e) {
-                                        return __fmul_rn(at(l), __fadd_rn(e.x, __fmul_rn(w, e.y)));
-                                    };
-                                    int l = loc0;
-                                    float acc4[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 2
-                                    for (; l + 3 < loc1; l += 4, a += 4 * 256)
-                                    {
-                                        acc4[0] = __fadd_rn(acc4[0], tap(l, pair_at<0>(a)));
-                                        acc4[1] = __fadd_rn(acc4[1], tap(l + 1, pair_at<256>(a)));
-                                        acc4[2] = __fadd_rn(acc4[2], tap(l + 2, pair_at<512>(a)));
-                                        acc4[3] = __fadd_rn(acc4[3], tap(l + 3, pair_at<768>(a)));
-                                    }
-                                    float accum = __fadd_rn(__fadd_rn(acc4[0], acc4[2]), __fadd_rn(acc4[1], acc4[3]));
-                                    for (; l < loc1; ++l, a += 256) accum = __fadd_rn(accum, tap(l, pair_at<0>(a)));
-                                    return accum;
-                                };
+                                auto taps = [&](auto at) { return mono_taps(win, at, loc0, loc1, inPos); };
+                                auto taps_exact = [&](auto at) { return mono_taps_exact(win, at, loc0, loc1, inPos); };
                                 auto run = [&](auto at) {
                                     if constexpr (kPairs && kMagic && kFma)
                                         if (exact) return taps_exact(at);
@@ -472,25 +498,7 @@ __global__ void __launch_bounds__(kThreads, 4)
                                 *RPPB_WR(y + outPos) = r;
                             }
                             else
-                            {
-                                constexpr int kMaxC = 16;
-                                float acc[kMaxC];
-#pragma unroll
-                                for (int c = 0; c < kMaxC; ++c) acc[c] = 0.f;
-                                float xx = __fsub_rn(float(loc0), inPos);
-                                for (int l = loc0; l < loc1; ++l, xx = __fadd_rn(xx, 1.f))
-                                {
-                                    const float wv = win.scalar(xx);
-#pragma unroll
-                                    for (int c = 0; c < kMaxC; ++c)
-                                        if (c < C)
-                                            acc[c] = __fadd_rn(acc[c],
-                                                               __fmul_rn(__ldg(RPPB_RD(in + (long long)l * C + c)), wv));
-                                }
-#pragma unroll
-                                for (int c = 0; c < kMaxC; ++c)
-                                    if (c < C) *RPPB_WR(y + ((long long)outPos * C + c)) = acc[c];
-                            }
+                                channel_taps(win, in, y + (long long)outPos * C, C, loc0, loc1, inPos);
                         }
                         if (kMix) __syncwarp();   // the warp's span is restaged by its next slice
                     }
@@ -502,15 +510,468 @@ __global__ void __launch_bounds__(kThreads, 4)
     }
 }
 
+// ---------------------------------------------------------------- held weights (16 lobes)
+// The weights of an output's 32 taps depend on its phase alone, and a block's phases follow from its first
+// one, so blocks whose first phase has the same bits share all 256 x 32 weights.  For integer rates the first
+// phase repeats every P = outRate / gcd(256 inRate, outRate) blocks (5 for 44.1 or 22.05 kHz to 16 kHz, 1 for
+// 48 kHz); the FP64 block origin can move it by a rounding, so the bits are compared block by block.  A CTA
+// takes an item of up to kItemBlocks blocks P apart, computes the weights once with the reference's
+// operations, holds them in registers and runs every block of the item through them: one sample load and
+// two float operations per tap instead of two loads and four (or, outside the exact walk, ten) operations.
+//
+// Four lanes share an output: lane q sums the taps q, q + 4, ..., the reference's SSE lane q, and two
+// exchanges fold the sums as (l0 + l2) + (l1 + l3).  A warp's 32 sample loads then cover the span of 8
+// neighbouring outputs, 8 ratio + 4 consecutive floats: no bank conflicts up to a ratio of 3.5, where lanes on
+// neighbouring outputs (stride ratio) take 2 to 3 shared-memory wavefronts per load.  A thread holds 4
+// outputs' quarters, 32 weights (2 outputs and twice the threads: the per-block work of a thread, staging and
+// addresses, is then as large as its sums).  The next block's span is loaded into registers while the current
+// one is summed.  Blocks whose taps reach past the signal's ends, or whose first phase differs, take the
+// reference's operations output by output.
+constexpr int kHeldLobes = 16;
+constexpr int kItemBlocks = 16;      // blocks of an item
+constexpr int kHeldCtas = 2;         // per SM
+constexpr int kHeldSpan = 1024;      // staged samples of a block: ratios up to 3.8
+constexpr int kHeldPeriod = 64;      // longer periods share nothing: items of one block
+constexpr int kHeldWarps = 8;        // compute warps: 8 outputs per pass and warp, four passes per block
+constexpr int kHeldCompute = kHeldWarps * 32, kHeldThreads = kHeldCompute + 32;
+constexpr int kHeldOuts = kBlock / (kHeldWarps * 8);   // outputs per thread
+constexpr int kSpanLoads = kHeldSpan / kHeldCompute;
+static_assert(kHeldOuts == 4, "the fold of the lane sums assumes four outputs per thread");
+
+__device__ __forceinline__ int phase_period(float inRate, float outRate)
+{
+    const bool whole = inRate >= 1.f && outRate >= 1.f && inRate <= 1048576.f && outRate <= 1048576.f &&
+                       inRate == floorf(inRate) && outRate == floorf(outRate);
+    if (!whole) return 0;
+    const int o = int(outRate);
+    int a = int(inRate) * kBlock, b = o;   // at most 2^28
+    while (b)
+    {
+        const int t = a % b;
+        a = b;
+        b = t;
+    }
+    const int p = o / a;
+    return p <= kHeldPeriod ? p : 0;
+}
+
+// How a resampled sample's blocks are dealt to items: item i takes blocks i % period + period * (first + j).
+struct ItemPlan
+{
+    int blocks, period, per, groups;
+    __device__ __forceinline__ ItemPlan(int outEnd, float inRate, float outRate)
+    {
+        blocks = (outEnd + kBlock - 1) / kBlock;
+        const int p = phase_period(inRate, outRate);
+        period = p == 0 ? 1 : max(1, min(p, blocks));
+        const int each = (blocks + period - 1) / period;
+        groups = p == 0 ? each : (each + kItemBlocks - 1) / kItemBlocks;
+        per = groups > 0 ? (each + groups - 1) / groups : 0;
+    }
+    __device__ __forceinline__ long long items() const { return (long long)period * groups; }
+};
+
+struct HeldCount
+{
+    const float* inRate;
+    const float* outRate;
+    const int* dims;
+    bool mix;
+    __device__ long long operator()(int b) const
+    {
+        const int L = *RPPB_RD(dims + 2 * b), Cs = *RPPB_RD(dims + (2 * b + 1));
+        const float ir = *RPPB_RD(inRate + b), orr = *RPPB_RD(outRate + b);
+        if (L <= 0 || Cs <= 0) return 0;
+        if (ir == orr) return ((long long)L * (mix ? 1 : Cs) + kCopyChunk - 1) / kCopyChunk;
+        const int outEnd = out_length(L, ir, orr);
+        return outEnd <= 0 ? 0 : ItemPlan(outEnd, ir, orr).items();
+    }
+};
+
+constexpr int kBlockHeld = 0, kBlockEdge = 1, kBlockOther = 2;
+struct HeldItem
+{
+    const float* x;
+    float* y;
+    int L, Csrc, C, unit;      // unit: copies only
+    int mode;                  // kUnitSkip, kUnitCopy or kUnitResample; -1: no item left
+    int count, held;           // blocks; the first `held` of them share the item's weights
+    int lo, span;              // the blocks' samples are [origin + lo, origin + lo + span)
+    float wc;
+    float fscale;
+    int block[kItemBlocks];    // output block
+    int origin[kItemBlocks];   // the input sample its phases count from
+    int outs[kItemBlocks];     // its outputs
+    int kind[kItemBlocks];
+    float first[kItemBlocks];  // its first phase
+};
+
+// The reference's phase sum of a block.
+__device__ __forceinline__ void block_phases(float p, float fscale, float* to)
+{
+    float4* out = reinterpret_cast<float4*>(to);
+#pragma unroll 8
+    for (int k = 0; k < kBlock / 4; ++k)
+    {
+        float4 q;
+        q.x = p;
+        q.y = p = __fadd_rn(p, fscale);
+        q.z = p = __fadd_rn(p, fscale);
+        q.w = p = __fadd_rn(p, fscale);
+        p = __fadd_rn(p, fscale);
+        out[k] = q;
+    }
+}
+
+// The item's blocks that do not share its weights, an output per thread with the reference's operations.  Not
+// inlined: its registers would come on top of the held weights.
+template <bool kMix>
+__device__ RPPB_OUT_OF_LINE void other_blocks(const Win<true, true, true>& win, const HeldItem& it, const MonoMix& mix,
+                                          const float* ph, float* s_other, int exactMinE, int exactMaxE)
+{
+    for (int e = it.held; e < it.count; ++e)
+    {
+        const float* phase = ph;
+        if (it.kind[e] == kBlockOther)
+        {
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+            if (threadIdx.x == 0) block_phases(it.first[e], it.fscale, s_other);
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+            phase = s_other;
+        }
+        const int k = threadIdx.x;
+        if (k >= it.outs[e]) continue;
+        const float p = phase[k];
+        const int origin = it.origin[e], L = it.L, C = it.C;
+        const int xc = int(ceilf(p));
+        int loc0 = xc - kHeldLobes, loc1 = xc + kHeldLobes;
+        if (loc0 + origin < 0) loc0 = -origin;
+        if (loc1 + origin > L) loc1 = L - origin;
+        const long long outPos = (long long)it.block[e] * kBlock + k;
+        if (kMix || C == 1)
+        {
+            auto at = [&](int l) {
+                return kMix ? mix((long long)origin + l) : __ldg(RPPB_RD(it.x + ((long long)origin + l)));
+            };
+            const int ex = int((__float_as_uint(p) >> 23) & 0xffu) - 127;
+            *RPPB_WR(it.y + outPos) = ex >= exactMinE && ex <= exactMaxE ? mono_taps_exact(win, at, loc0, loc1, p)
+                                                                         : mono_taps(win, at, loc0, loc1, p);
+        }
+        else
+            channel_taps(win, it.x + (long long)origin * C, it.y + outPos * C, C, loc0, loc1, p);
+    }
+}
+
+template <bool kMix>
+__global__ void __launch_bounds__(kHeldThreads, 2)
+    resample_held_kernel(const float* __restrict__ src, uint32_t srcStride, float* __restrict__ dst, uint32_t dstStride,
+                         const float* __restrict__ inRateT, const float* __restrict__ outRateT,
+                         const int* __restrict__ dims, ResampleWindowDev wd, bool normalize,
+                         const long long* __restrict__ prefix, unsigned long long* __restrict__ nextItem, int n)
+{
+    extern __shared__ float s_lut[];   // the padded (value, next - value) table, then two staged spans
+    const int pairCount = int(resample_pair_entries(wd.lutSize, wd.padLeft, wd.padRight));
+    float* s_span = s_lut + 2 * pairCount;
+    __shared__ __align__(16) float s_phase[2][kBlock];
+    __shared__ __align__(16) float s_other[kBlock];   // phases of a block of kind kBlockOther
+    __shared__ HeldItem s_item[2];
+    for (int i = threadIdx.x; i < pairCount; i += kHeldThreads)
+    {
+        const int e = min(max(i - wd.padLeft, 0), wd.lutSize - 2);
+        const float v0 = *RPPB_RD(wd.lut + e), v1 = *RPPB_RD(wd.lut + (e + 1));
+        reinterpret_cast<float2*>(s_lut)[i] = make_float2(v0, __fsub_rn(v1, v0));
+    }
+    const float2* pairs = reinterpret_cast<const float2*>(s_lut) + wd.padLeft;
+    const Win<true, true, true> win{s_lut, pairs, wd.lutSize, wd.scale, wd.center,
+                                    uint32_t(__cvta_generic_to_shared(pairs)) - 0x5A000000u};
+    __shared__ long long s_prefix[kPrefixCache];
+    grid_dependency_wait();   // the prefix and the zeroed counter
+    nextItem = dependency_result(nextItem);
+    prefix = cache_prefix(dependency_result(prefix), n, s_prefix);
+    const long long total = prefix[n];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+    // the phase warp claims the next item and decodes it into slot
+    auto decode = [&](int slot) {
+        HeldItem& it = s_item[slot];
+        long long w = 0;
+        if (lane == 0) w = (long long)atomicAdd(RPPB_WR(nextItem), 1ull);
+        w = __shfl_sync(0xffffffffu, w, 0);
+        if (w >= total)
+        {
+            if (lane == 0) it.mode = -1;
+            return;
+        }
+        const int b = ragged_find(prefix, n, w);
+        const int local = int(w - prefix[b]);
+        const int L = *RPPB_RD(dims + 2 * b), Csrc = *RPPB_RD(dims + (2 * b + 1)), C = kMix ? 1 : Csrc;
+        const float inRate = *RPPB_RD(inRateT + b), outRate = *RPPB_RD(outRateT + b);
+        const float* x = src + size_t(b) * srcStride;
+        const int mode = inRate == outRate ? kUnitCopy : (kMix && Csrc > 64) ? kUnitSkip : kUnitResample;
+        if (lane == 0)
+        {
+            it.x = x;
+            it.y = dst + size_t(b) * dstStride;
+            it.L = L;
+            it.Csrc = Csrc;
+            it.C = C;
+            it.unit = local;
+            it.mode = mode;
+            it.wc = kMix ? MonoMix::weight(max(Csrc, 1), normalize) : 1.f;
+        }
+        if (mode != kUnitResample) return;
+        const int outFull = out_length(L, inRate, outRate);
+        const int outEnd = min(outFull, int(dstStride / uint32_t(C)));
+        const ItemPlan plan(outFull, inRate, outRate);
+        const double scale = __ddiv_rn(double(inRate), double(outRate));
+        const float fscale = __double2float_rn(scale);
+        const int residue = local % plan.period, j0 = local / plan.period * plan.per;
+        // lane j: the item's block j
+        const int u = residue + plan.period * (j0 + lane);
+        const bool mine = lane < plan.per && u < plan.blocks && u * kBlock < outEnd;
+        const double raw = __dmul_rn(double(u * kBlock), scale);
+        const int origin = int(raw);
+        const float first = __double2float_rn(__dsub_rn(raw, double(origin)));
+        const unsigned all = __ballot_sync(0xffffffffu, mine);
+        const int count = __popc(all);
+        const float held = __shfl_sync(0xffffffffu, first, 0);
+        if (lane == 0) block_phases(held, fscale, s_phase[slot]);
+        __syncwarp();
+        const float* ph = s_phase[slot];
+        const int lo = int(ceilf(ph[0])) - kHeldLobes, span = int(ceilf(ph[kBlock - 1])) + kHeldLobes - lo;
+        if (mine)
+        {
+            const int outs = min(kBlock, outEnd - u * kBlock);
+            const long long from = (long long)origin + lo;
+            const long long to = (long long)origin + int(ceilf(ph[outs - 1])) + kHeldLobes;
+            const int kind = __float_as_uint(first) != __float_as_uint(held)              ? kBlockOther
+                             : from < 0 || to > L || span > kHeldSpan || (!kMix && C != 1) ? kBlockEdge
+                                                                                           : kBlockHeld;
+            // the blocks that share the weights first
+            const unsigned share = __ballot_sync(all, kind == kBlockHeld);
+            const unsigned before = (1u << lane) - 1u;
+            const int at = kind == kBlockHeld ? __popc(share & before) : __popc(share) + __popc(all & ~share & before);
+            it.block[at] = u;
+            it.origin[at] = origin;
+            it.outs[at] = outs;
+            it.first[at] = first;
+            it.kind[at] = kind;
+            if (lane == 0) it.held = __popc(share);
+            // ask L2 for the block's samples an item ahead of their use
+            const long long f = max(from, 0ll), t = min(to, (long long)L);
+            if (t > f) l2_prefetch(x + f * Csrc, x + t * Csrc);
+        }
+        if (lane == 0)
+        {
+            it.count = count;
+            if (count == 0) it.held = 0;
+            it.lo = lo;
+            it.span = span;
+            it.fscale = fscale;
+        }
+    };
+
+    if (threadIdx.x == 0) s_item[0].mode = kUnitSkip;   // the first pass only decodes
+    __syncthreads();
+    for (int cur = 0;; cur ^= 1)
+    {
+        const HeldItem& it = s_item[cur];
+        const int mode = it.mode;
+        if (mode < 0) break;
+        if (warp == kHeldWarps) decode(cur ^ 1);
+        else if (mode == kUnitCopy)
+        {
+            const MonoMix mix{it.x, kMix ? it.Csrc : 1, it.wc};
+            const long long L = it.L;
+            const long long count = kMix ? min(L, (long long)dstStride) : min(L * it.C, (long long)min(srcStride, dstStride));
+            const long long i0 = (long long)it.unit * kCopyChunk, end = min(count, i0 + kCopyChunk);
+            const float* x = it.x;
+            float* y = it.y;
+            for (long long i = i0 + threadIdx.x; i < end; i += 4 * kHeldCompute)
+            {
+                float v[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (i + k * kHeldCompute < end) v[k] = kMix ? mix(i + k * kHeldCompute) : *RPPB_RD(x + (i + k * kHeldCompute));
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (i + k * kHeldCompute < end) *RPPB_WR(y + (i + k * kHeldCompute)) = v[k];
+            }
+        }
+        else if (mode == kUnitResample)
+        {
+            const int q = lane & 3, o8 = lane >> 2, tid = threadIdx.x;
+            const float* ph = s_phase[cur];
+            const MonoMix mix{it.x, kMix ? it.Csrc : 1, it.wc};
+            const int held = it.held;
+            if (held > 0)
+            {
+                const int lo = it.lo, span = it.span;
+                // a block's samples: loaded into registers, then stored (down-mixed) into a span buffer
+                const int channels = kMix ? it.Csrc : 1;
+                const bool two = channels == 2 && (reinterpret_cast<uintptr_t>(it.x) & 7) == 0;
+                const float wc = it.wc;
+                const float* base = it.x + (long long)(lo + tid) * (two ? 2 : 1);
+                float2 v[kSpanLoads];
+                auto load = [&](int j) {
+                    const int origin = it.origin[j];
+                    const int most = min(span, it.L - origin - lo) - tid;   // samples past the signal are not summed
+                    if (two)
+                    {
+                        const float2* at = reinterpret_cast<const float2*>(base) + origin;
+#pragma unroll
+                        for (int k = 0; k < kSpanLoads; ++k)
+                            if (k * kHeldCompute < most) v[k] = __ldg(RPPB_RD(at + k * kHeldCompute));
+                    }
+                    else if (channels == 1)
+                    {
+                        const float* at = base + origin;
+#pragma unroll
+                        for (int k = 0; k < kSpanLoads; ++k)
+                            if (k * kHeldCompute < most) v[k].x = __ldg(RPPB_RD(at + k * kHeldCompute));
+                    }
+                    else
+                    {
+#pragma unroll
+                        for (int k = 0; k < kSpanLoads; ++k)
+                            if (k * kHeldCompute < most) v[k].x = mix((long long)origin + lo + tid + k * kHeldCompute);
+                    }
+                };
+                auto store = [&](int slot) {
+                    float* to = s_span + slot * kHeldSpan + tid;
+                    if (two)
+                    {
+                        // MonoMix's sum for two channels
+#pragma unroll
+                        for (int k = 0; k < kSpanLoads; ++k)
+                            if (tid + k * kHeldCompute < span)
+                                to[k * kHeldCompute] = __fadd_rn(__fadd_rn(0.f, __fmul_rn(v[k].x, wc)), __fmul_rn(v[k].y, wc));
+                    }
+                    else
+                    {
+#pragma unroll
+                        for (int k = 0; k < kSpanLoads; ++k)
+                            if (tid + k * kHeldCompute < span) to[k * kHeldCompute] = v[k].x;
+                    }
+                };
+                load(0);
+                // weights of taps q, q + 4, ... of outputs m * 64 + warp * 8 + o8
+                float w[kHeldOuts][8];
+                int off[kHeldOuts];
+#pragma unroll
+                for (int m = 0; m < kHeldOuts; ++m)
+                {
+                    const float p = ph[m * 64 + warp * 8 + o8];
+                    const int l = int(ceilf(p)) - kHeldLobes;
+                    off[m] = l - lo + q;
+                    const float begin = __fsub_rn(float(l), p);
+                    const int e = int((__float_as_uint(p) >> 23) & 0xffu) - 127;
+                    if (__all_sync(0xffffffffu, e >= wd.exactMinE && e <= wd.exactMaxE))
+                    {
+                        // the exact walk: one entry and weight, then 32 entries per tap
+                        constexpr float kM = 12582912.0f;   // 1.5 * 2^23
+                        const float raw = __fmaf_rn(begin, win.scale, win.center);
+                        const float r = __fadd_rd(raw, kM);
+                        const float f = __fsub_rn(raw, __fsub_rn(r, kM));
+                        const uint32_t a = win.bias + (uint32_t(__float_as_int(r)) << 3) + 256u * q;
+                        auto at = [&](float2 e) { return __fadd_rn(e.x, __fmul_rn(f, e.y)); };
+                        w[m][0] = at(pair_at<0>(a));
+                        w[m][1] = at(pair_at<1024>(a));
+                        w[m][2] = at(pair_at<2048>(a));
+                        w[m][3] = at(pair_at<3072>(a));
+                        w[m][4] = at(pair_at<4096>(a));
+                        w[m][5] = at(pair_at<5120>(a));
+                        w[m][6] = at(pair_at<6144>(a));
+                        w[m][7] = at(pair_at<7168>(a));
+                    }
+                    else
+                    {
+                        float t = __fadd_rn(begin, float(q));
+#pragma unroll
+                        for (int k = 0; k < 8; ++k, t = __fadd_rn(t, 4.f)) w[m][k] = win.lane(t);
+                    }
+                }
+                const bool up = q & 2, odd = q & 1;
+                const int mine = q * 64 + warp * 8 + o8;   // the output this lane ends with
+                float* y = it.y + mine;
+                store(0);
+                asm volatile("bar.sync 1, 256;" ::: "memory");
+                for (int j = 0; j < held; ++j)
+                {
+                    if (j + 1 < held) load(j + 1);
+                    const float* sp = s_span + (j & 1) * kHeldSpan;
+                    float acc[kHeldOuts];
+#pragma unroll
+                    for (int m = 0; m < kHeldOuts; ++m)
+                    {
+                        const float* s = sp + off[m];
+                        acc[m] = 0.f;
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) acc[m] = __fadd_rn(acc[m], __fmul_rn(s[4 * k], w[m][k]));
+                    }
+                    // fold (l0 + l2) + (l1 + l3): after the exchanges lane q has output q * 64 + warp * 8 + o8
+                    const float g0 = __shfl_xor_sync(0xffffffffu, up ? acc[0] : acc[2], 2);
+                    const float g1 = __shfl_xor_sync(0xffffffffu, up ? acc[1] : acc[3], 2);
+                    const float h0 = __fadd_rn(up ? acc[2] : acc[0], g0), h1 = __fadd_rn(up ? acc[3] : acc[1], g1);
+                    const float r = __fadd_rn(odd ? h1 : h0, __shfl_xor_sync(0xffffffffu, odd ? h0 : h1, 1));
+                    if (mine < it.outs[j]) *RPPB_WR(y + (long long)it.block[j] * kBlock) = r;
+                    if (j + 1 < held) store((j + 1) & 1);
+                    asm volatile("bar.sync 1, 256;" ::: "memory");
+                }
+            }
+            if (held < it.count) other_blocks<kMix>(win, it, mix, ph, s_other, wd.exactMinE, wd.exactMaxE);
+        }
+        __syncthreads();   // slot cur is free, slot cur ^ 1 is ready
+    }
+}
+
 }  // namespace
+
+namespace {
+
+// The held-weights kernel serves windows of 16 lobes with a power-of-two table scale (what kaiser_sinc and the
+// reference's own window give at 16 lobes), whatever the rates; other windows take resample_kernel.
+bool resample_held_ok(const ResampleWindowDev& w, bool magic, bool fma)
+{
+    return magic && fma && w.lobes == kHeldLobes &&
+           resample_smem_floats(w, true, true) * sizeof(float) <= kPairTableLimit;
+}
+
+template <bool kMix>
+void launch_held(Handle& h, void* scratch, const float* src, uint32_t srcStride, float* dst, uint32_t dstStride, int n,
+                 const float* inRate, const float* outRate, const int* dims, const ResampleWindowDev& w,
+                 bool normalize)
+{
+    const size_t smem = resample_smem_floats(w, true, true) * sizeof(float);   // the table and two spans
+    static_assert(kWarps * 256 == 2 * kHeldSpan, "resample_smem_floats counts the spans");
+    const int grid = persistent_grid(h, reinterpret_cast<const void*>(resample_held_kernel<kMix>), kHeldThreads, smem);
+    Carver cv(scratch);
+    long long* prefix = cv.take<long long>(n + 1);
+    unsigned long long* next = cv.take<unsigned long long>(1);
+    launch_ragged_prefix(HeldCount{inRate, outRate, dims, kMix}, n, prefix, h.stream(),
+                         reinterpret_cast<unsigned*>(next), 2);
+    launch_dependent(resample_held_kernel<kMix>, dim3(grid), dim3(kHeldThreads), smem, h.stream(),
+                     "resample_held_kernel", src, srcStride, dst, dstStride, inRate, outRate, dims, w, normalize,
+                     static_cast<const long long*>(prefix), next, n);
+    count_launch();
+}
+
+}  // namespace
+
+size_t resample_scratch_bytes(int n)
+{
+    Carver cv(nullptr);
+    cv.take<long long>(n + 1);
+    cv.take<unsigned long long>(1);
+    return cv.used();
+}
 
 void launch_resample(Handle& h, void* scratch, const float* src, uint32_t srcStride, float* dst, uint32_t dstStride,
                      int n, const float* inRate, const float* outRate, const int* dims, const ResampleWindowDev& win,
-                     bool downmix, bool normalize)
+                     int channels, bool downmix, bool normalize)
 {
     if (n <= 0) return;
     long long* prefix = static_cast<long long*>(scratch);
-    launch_ragged_prefix(ResampleCount{inRate, outRate, dims, downmix, nullptr, 0.f}, n, prefix, h.stream());
     ResampleWindowDev w = win;
     resample_pads(w);
     const bool pairs = w.padLeft >= 0 && resample_smem_floats(w, true, downmix) * sizeof(float) <= kPairTableLimit;
@@ -518,6 +979,20 @@ void launch_resample(Handle& h, void* scratch, const float* src, uint32_t srcStr
     const bool magic = resample_magic_ok(w, pairs);
     const bool fma = resample_scale_pow2(w);
     resample_exact_range(w, magic, fma);
+    // The held-weights kernel pays from four full items per CTA on, by the batch's padded size: at 2 CTAs per SM
+    // 18944 blocks, 5 minutes at 16 kHz (clips of 3 s, mono / stereo: 32 clips 32 against 33 us and 45 against 38,
+    // 64 clips 43 against 52 us and 61 against 62, and 64 clips of 6 s 73 against 112 us).
+    const long long padded = (long long)n * ((dstStride + kBlock - 1) / kBlock);
+    const bool many = padded >= 4ll * kItemBlocks * kHeldCtas * h.num_sms();
+    if (many && (downmix || channels <= 1) && resample_held_ok(w, magic, fma))
+    {
+        if (downmix)
+            launch_held<true>(h, scratch, src, srcStride, dst, dstStride, n, inRate, outRate, dims, w, normalize);
+        else
+            launch_held<false>(h, scratch, src, srcStride, dst, dstStride, n, inRate, outRate, dims, w, normalize);
+        return;
+    }
+    launch_ragged_prefix(ResampleCount{inRate, outRate, dims, downmix, nullptr, 0.f}, n, prefix, h.stream());
     auto go = [&](auto kernel) {
         const int grid = persistent_grid(h, reinterpret_cast<const void*>(kernel), kThreads, smem);
         kernel<<<grid, kThreads, smem, h.stream()>>>(src, srcStride, dst, dstStride, inRate, outRate, dims, w,
@@ -540,7 +1015,6 @@ void launch_resample_clips(Handle& h, void* scratch, const RppbClip* clips, int 
 {
     if (n <= 0) return;
     long long* prefix = static_cast<long long*>(scratch);
-    launch_ragged_prefix(ResampleCount{nullptr, nullptr, nullptr, false, clips, outRate}, n, prefix, h.stream());
     ResampleWindowDev w = win;
     resample_pads(w);
     const bool pairs = w.padLeft >= 0 && resample_smem_floats(w, true, false) * sizeof(float) <= kPairTableLimit;
@@ -548,6 +1022,7 @@ void launch_resample_clips(Handle& h, void* scratch, const RppbClip* clips, int 
     const bool magic = resample_magic_ok(w, pairs);
     const bool fma = resample_scale_pow2(w);
     resample_exact_range(w, magic, fma);
+    launch_ragged_prefix(ResampleCount{nullptr, nullptr, nullptr, false, clips, outRate}, n, prefix, h.stream());
     auto go = [&](auto kernel) {
         const int grid = persistent_grid(h, reinterpret_cast<const void*>(kernel), kThreads, smem);
         kernel<<<grid, kThreads, smem, h.stream()>>>(nullptr, 0, nullptr, 0, nullptr, nullptr, nullptr, w, false,
