@@ -1420,9 +1420,14 @@ extern "C" SHARED_PUBLIC RppStatus rppt_normalize_gpu(RppPtr_t srcPtr, RpptGener
         const int n = int(dd.dims[0]);
         if (n <= 0) return RPP_SUCCESS;
         const int compute = computeMeanStddev & 3;
+        // both statistics per contiguous row: one kernel, no task list
+        void *meanDirect = nullptr, *stdDirect = nullptr;
+        const bool rowwise = axisMask == 2 && compute == 3 && sd.strides[2] == 1 &&
+                             normalize_rows_fit(int(std::min<uint32_t>(sd.dims[2], INT32_MAX))) &&
+                             h.device_writable(meanTensor, &meanDirect) && h.device_writable(stdDevTensor, &stdDirect);
         // roi lengths are needed on the host (parameter counts, work list)
         const std::vector<uint32_t> roi = roi_to_host(h, roiTensor, size_t(n) * 4);
-        int maxSize = 1;
+        int maxSize = 1, maxCount = 0;
         std::vector<NormalizeSample> samples(n);
         std::vector<int4> tasks;
         for (int b = 0; b < n; ++b)
@@ -1458,7 +1463,8 @@ extern "C" SHARED_PUBLIC RppStatus rppt_normalize_gpu(RppPtr_t srcPtr, RpptGener
                 params = s.len0;
             }
             s.normFactor = float(1.0 / double(s.count));
-            if (compute)
+            maxCount = std::max(maxCount, s.count);
+            if (compute && !rowwise)
             {
                 if (s.count >= kNormalizeWarpMinElems)
                     for (int p = 0; p < params; ++p) tasks.push_back(make_int4(b, p, 1, 1));
@@ -1467,6 +1473,39 @@ extern "C" SHARED_PUBLIC RppStatus rppt_normalize_gpu(RppPtr_t srcPtr, RpptGener
             }
         }
         const size_t perAll = size_t(n) * maxSize;
+        NormalizeArgs a;
+        a.src = reinterpret_cast<const float*>(static_cast<const char*>(srcPtr) + sd.offsetInBytes);
+        a.dst = reinterpret_cast<float*>(static_cast<char*>(dstPtr) + dd.offsetInBytes);
+        a.n = n;
+        a.srcStride0 = sd.strides[0];
+        a.srcStride1 = sd.strides[1];
+        a.srcStride2 = sd.strides[2];
+        a.dstStride0 = dd.strides[0];
+        a.dstStride1 = dd.strides[1];
+        if (a.dstStride1 == 0) return RPP_ERROR_INVALID_ARGUMENTS;
+        a.axisMask = axisMask;
+        a.compute = compute;
+        a.scale = scale;
+        a.shift = shift;
+        a.maxSize = maxSize;
+        a.meanIn = nullptr;
+        if (rowwise)
+        {
+            // the statistics go straight to the caller's arrays (entries past a sample's parameter count keep
+            // the caller's values, as in the reference)
+            Carver m(nullptr);
+            m.take<NormalizeSample>(n);
+            NormalizeSample* dSamples = static_cast<NormalizeSample*>(h.workspace(m.used()));
+            h.upload(dSamples, samples.data(), samples.size() * sizeof(NormalizeSample));
+            a.samples = dSamples;
+            a.meanOut = static_cast<float*>(meanDirect);
+            a.invOut = static_cast<float*>(stdDirect);
+            check_tensors(h, srcPtr, sd, dstPtr, dd, n);
+            h.check_add(meanDirect, perAll * sizeof(float), true);
+            h.check_add(stdDirect, perAll * sizeof(float), true);
+            launch_normalize_rows(h, a, maxCount);
+            return RPP_SUCCESS;
+        }
         const size_t meanInCount = compute == 0 ? size_t(maxSize) : perAll;
         Carver m(nullptr);
         m.take<NormalizeSample>(n);
@@ -1486,21 +1525,6 @@ extern "C" SHARED_PUBLIC RppStatus rppt_normalize_gpu(RppPtr_t srcPtr, RpptGener
         float* stdStage = cv.take<float>(meanInCount);
         h.upload(dSamples, samples.data(), samples.size() * sizeof(NormalizeSample));
         if (!tasks.empty()) h.upload(dTasks, tasks.data(), tasks.size() * sizeof(int4));
-        NormalizeArgs a;
-        a.src = reinterpret_cast<const float*>(static_cast<const char*>(srcPtr) + sd.offsetInBytes);
-        a.dst = reinterpret_cast<float*>(static_cast<char*>(dstPtr) + dd.offsetInBytes);
-        a.n = n;
-        a.srcStride0 = sd.strides[0];
-        a.srcStride1 = sd.strides[1];
-        a.srcStride2 = sd.strides[2];
-        a.dstStride0 = dd.strides[0];
-        a.dstStride1 = dd.strides[1];
-        if (a.dstStride1 == 0) return RPP_ERROR_INVALID_ARGUMENTS;
-        a.axisMask = axisMask;
-        a.compute = compute;
-        a.scale = scale;
-        a.shift = shift;
-        a.maxSize = maxSize;
         a.samples = dSamples;
         a.meanIn = (compute & 1) ? nullptr
                                  : static_cast<const float*>(h.device_view(meanTensor, meanInCount * 4, meanStage));

@@ -214,6 +214,10 @@ void launch_normalize(Handle& h, const NormalizeArgs& a, const int4* tasks, int 
                       const float* invEff, int paramOffsetPerSample, const float* stdToInvert, float* invertOut,
                       int invertCount);
 
+// Both statistics per contiguous row (axisMask 2, srcStride2 1), each row read once; maxCount = the longest row.
+bool normalize_rows_fit(int maxCount);
+void launch_normalize_rows(Handle& h, const NormalizeArgs& a, int maxCount);
+
 // normalize, every other type and rank (normalize_nd.cu): per-sample plans built by the dispatch.
 constexpr int kNormF32 = 0, kNormF16 = 1, kNormU8 = 2, kNormI8 = 3;
 struct NormNdLevel
