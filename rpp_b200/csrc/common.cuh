@@ -199,6 +199,21 @@ __device__ __forceinline__ float key_float(unsigned k)
     return __uint_as_float(u);
 }
 
+// multiplier * log2(max(minRatio, x * inv)) with the hardware base-2 logarithm.  kNormal: minRatio is a normal
+// number, so the argument is one too and the logarithm needs no scaling of subnormal arguments (same bits,
+// four instructions less).
+template <bool kNormal>
+__device__ __forceinline__ float decibel(float x, float inv, float minRatio, float multiplier)
+{
+    float t = __fmul_rn(x, inv);
+    t = minRatio < t ? t : minRatio;
+    float l;
+    if constexpr (kNormal) asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(t));
+    else l = __log2f(t);
+    return __fmul_rn(multiplier, l);
+}
+constexpr float kMinNormal = 1.17549435e-38f;
+
 __device__ __forceinline__ float warp_max(float v)
 {
 #pragma unroll

@@ -24,15 +24,25 @@
 #include <algorithm>
 #include <cstring>
 #include <string>
+#include <type_traits>
 
 #include "common.cuh"
 #include "fused_queue.cuh"
 #include "mel_tables.cuh"
 #include "ops.hpp"
 #include "stft.cuh"
+#include "stft_pair.cuh"
 
 namespace rppb {
 namespace {
+
+// The thread's index, read again where it is asked for.
+__device__ __forceinline__ int thread_index()
+{
+    int t;
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
+    return t;
+}
 
 template <int NFFT, int TFX>
 __global__ void __launch_bounds__(kFusedThreads, (NFFT <= 512 ? 3 : 2)) frontend_kernel(FrontendArgs a, const float2* __restrict__ twiddle,
@@ -42,19 +52,26 @@ __global__ void __launch_bounds__(kFusedThreads, (NFFT <= 512 ? 3 : 2)) frontend
                                                                  int* __restrict__ errorWord,
                                                                  const uint4* __restrict__ melTables)
 {
+    constexpr bool kPairs = PairPlan<NFFT>::use;   // stft_pair.cuh
     using S = StftShape<NFFT, kFusedThreads, TFX>;
-    constexpr int TF = S::TF, LD = S::OUT_LD;
+    using P = PairShape<NFFT>;
+    constexpr int TF = S::TF;
+    constexpr int LD = kPairs ? 2 : S::OUT_LD;     // floats between a frame's consecutive bins
     extern __shared__ __align__(16) unsigned char smem[];
-    const FusedLayout<NFFT, TFX> lay(a.mel.numFilter, a.W, a.hop);
+    const FusedLayout<NFFT, TFX, kPairs> lay(a.mel.numFilter, a.W, a.hop);
     float2* s_tw = reinterpret_cast<float2*>(smem + lay.tw);
     float2* s_tw1 = reinterpret_cast<float2*>(smem + lay.tw1);
     float* s_win = reinterpret_cast<float*>(smem + lay.win);
     float* s_span = reinterpret_cast<float*>(smem + lay.span);
     float2* s_fft = reinterpret_cast<float2*>(smem + lay.work);
-    float* s_out = reinterpret_cast<float*>(smem + lay.work + S::fft_bytes);
-    float2* melW = reinterpret_cast<float2*>(smem + lay.melW);   // bin k: (weight into filter i, into filter i - 1)
-    int2* melIv = reinterpret_cast<int2*>(smem + lay.melIv);     // interval i: bins [x, y)
-    int* melGrp = reinterpret_cast<int*>(smem + lay.melGrp);     // thread group g: filters [g], [g + 1])
+    float* s_out = reinterpret_cast<float*>(smem + lay.work + (kPairs ? 0 : S::fft_bytes));
+    __shared__ int s_mel[3];   // offsets of the mel tables: bin weights, intervals, thread groups
+    if (threadIdx.x == 0)
+    {
+        s_mel[0] = int(lay.melW);
+        s_mel[1] = int(lay.melIv);
+        s_mel[2] = int(lay.melGrp);
+    }
     __shared__ float s_warpMax[kFusedThreads / 32];
     const int nmel = a.mel.numFilter;
 
@@ -64,8 +81,6 @@ __global__ void __launch_bounds__(kFusedThreads, (NFFT <= 512 ? 3 : 2)) frontend
     // instead of 48; 263 -> 253 us on the 256-clip batch, bit-identical).
     for (int setupPass = 0, setupPasses = 1 + (a.n < 0); setupPass < setupPasses; ++setupPass)
     {
-        stft_tables<NFFT, kFusedThreads>(twiddle, a.window, a.W, s_tw, s_tw1, s_win, s_span);
-
         // the mel tables: copied from the handle's cache when the launch has them, else built here
         if (melTables)
         {
@@ -74,7 +89,11 @@ __global__ void __launch_bounds__(kFusedThreads, (NFFT <= 512 ? 3 : 2)) frontend
             __syncthreads();
         }
         else
-            build_fused_mel<NFFT, TFX>(a, smem, lay);
+            build_fused_mel<NFFT, TFX, kPairs>(a, smem, lay);   // its scratch may reach into the span buffer
+        if constexpr (kPairs)
+            stft_pair_tables<NFFT>(twiddle, a.window, a.W, s_tw, s_tw1, s_win, s_span);
+        else
+            stft_tables<NFFT, kFusedThreads>(twiddle, a.window, a.W, s_tw, s_tw1, s_win, s_span);
     }
 
     const int centerOffset = a.center ? a.W / 2 : 0;
@@ -85,9 +104,6 @@ __global__ void __launch_bounds__(kFusedThreads, (NFFT <= 512 ? 3 : 2)) frontend
     prefix = cache_prefix<kFusedPrefixCache>(dependency_result(prefix), nslots, s_prefix);
     const long long total = prefix[nslots];
     const SlotCount<TF> cnt{a, a.n, a.lookahead};
-    const int f = 2 * (threadIdx.x % (TF / 2));   // first of the two frame columns this thread owns in mel tiles
-    const int g = threadIdx.x / (TF / 2);
-
     // Thread 0 keeps two items decoded ahead in a two-entry ring (the claim's and the decode's
     // latencies overlap the current item) and asks L2 for each decoded spectrum item's input span
     // one item before it is staged; in the last 2 x grid items of the queue it reserves nothing
@@ -105,7 +121,10 @@ __global__ void __launch_bounds__(kFusedThreads, (NFFT <= 512 ? 3 : 2)) frontend
         const long long s1 = min((long long)n.L, (long long)last * a.hop - centerOffset + a.W);
         l2_prefetch(n.x + s0, n.x + s1);
     };
-    long long wAfter = 0;   // thread 0: the claimed item two after the current one (-1: none reserved)
+    // thread 0's: the claimed item two after the current one (-1: none reserved); kPairs: not in registers
+    __shared__ long long s_after;
+    long long r_after = 0;
+    long long& wAfter = kPairs ? s_after : r_after;
     int cur = 0;
     if (threadIdx.x == 0)
     {
@@ -117,68 +136,86 @@ __global__ void __launch_bounds__(kFusedThreads, (NFFT <= 512 ? 3 : 2)) frontend
         prefetch_span(s_it[1]);
     }
     __syncthreads();
+    // kPairs: whether the coming spectrum tile's samples are on their way into the span buffer (span_issue)
+    bool issued = false;
+    auto issue = [&](const Item& n, int f0) {
+        issued = span_issue<NFFT, true>(n.x, n.L, f0, n.F, a.W, a.hop, centerOffset, s_span);
+    };
+    if constexpr (kPairs)
+        if (s_it[0].kind == 0) issue(s_it[0], s_it[0].f0);
     for (;;)
     {
         // s_it[cur] is rewritten only after the barrier that ends this item's work
-        const Item it = s_it[cur];
-        if (it.kind < 0) break;
-        const int b = it.b;
-        const uint32_t hs = it.hs;
+        // (kPairs: read in place, its fields would cost registers across the transform)
+        const std::conditional_t<kPairs, const Item&, const Item> it = s_it[cur];
+        const int kind = it.kind, b = it.b;
+        if (kind < 0) break;
 
-        if (it.kind == 0)
+        if (kind == 0)
         {
             // subTiles tiles of TF frames; each tile's staging barrier also orders the previous
             // tile's mel reads of s_out before this tile's FFT overwrites it
-            const PreemphSource src{it.x, it.L, a.reflect, it.coeff, it.bval};
             float tmax = -FLT_MAX;
             for (int t = 0; t < a.subTiles; ++t)
             {
                 const int f0 = it.f0 + t * TF;
                 if (f0 >= it.F) break;   // uniform over the CTA
-                stft_tile<NFFT, kFusedThreads, TFX>(src, f0, it.F, a.W, a.hop, centerOffset, a.power, s_win, s_tw,
-                                                    s_tw1, s_span, s_fft, s_out);
+                const PreemphSource src{it.x, it.L, a.reflect, it.coeff, it.bval};
+                if constexpr (kPairs)
+                {
+                    span_arrive<NFFT>(issued, src, f0, it.F, a.W, a.hop, centerOffset, s_span);
+                    float2 z[P::R];
+                    if (issued) pair_gather<NFFT, true>(z, a.W, a.hop, s_win, s_span, it.coeff);
+                    else pair_gather<NFFT>(z, a.W, a.hop, s_win, s_span);
+                    __syncthreads();   // the span buffer is free: the next tile's samples travel from here on
+                    issued = false;
+                    if (t + 1 < a.subTiles && f0 + TF < it.F) issue(it, f0 + TF);
+                    else if (s_it[cur ^ 1].kind == 0) issue(s_it[cur ^ 1], s_it[cur ^ 1].f0);
+                    pair_transform<NFFT>(z, a.power, s_tw, s_tw1, s_out);
+                }
+                else
+                    stft_tile<NFFT, kFusedThreads, TFX>(src, f0, it.F, a.W, a.hop, centerOffset, a.power, s_win, s_tw, s_tw1,
+                                                  s_span, s_fft, s_out);
                 __syncthreads();
+                // first of the two frame columns this thread sums, its filters and their tables: found again for
+                // each tile, so that no register holds them across the transform
+                const int tid = kPairs ? thread_index() : int(threadIdx.x);
+                const int f = 2 * (tid % (TF / 2)), g = tid / (TF / 2);
+                if constexpr (kPairs) tmax = -FLT_MAX;   // folded tile by tile
                 if (f < it.F - f0)
                 {
-                    // one sweep over the group's intervals for frames f and f + 1; each power
-                    // pair is read once.  Scalar __fmul_rn / __fadd_rn: a paired multiply feeding
-                    // a paired add may be contracted into one rounding by the assembler.
+                    const float2* melW = reinterpret_cast<const float2*>(smem + (kPairs ? s_mel[0] : int(lay.melW)));
+                    const int2* melIv = reinterpret_cast<const int2*>(smem + (kPairs ? s_mel[1] : int(lay.melIv)));
+                    const int* melGrp = reinterpret_cast<const int*>(smem + (kPairs ? s_mel[2] : int(lay.melGrp)));
+                    const float* s_pow = kPairs ? s_out + (f >> 1) * P::PAIR_FLOATS : s_out + f;   // bin 0
+                    // one sweep over the group's intervals for frames f and f + 1
                     const bool second = f + 1 < it.F - f0;
+                    const uint32_t hs = it.hs;
                     const int m0 = melGrp[g], m1 = melGrp[g + 1];
                     float* yp = it.y + size_t(f0 - it.f0) + size_t(m0) * hs + f;
-                    float2 fall = make_float2(0.f, 0.f);   // filter i - 1: rising sum, then falling terms
-                    for (int i = m0; i <= m1; ++i)
-                    {
-                        const int2 iv = melIv[i];
-                        const float* sp = s_out + iv.x * LD + f;
-                        float2 rise = make_float2(0.f, 0.f);   // filter i
-#pragma unroll 1
-                        for (int k = iv.x; k < iv.y; ++k, sp += LD)
+                    mel_sweep<LD>(s_pow, melW, melIv, m0, m1, [&](float2 v) {
+                        *RPPB_WR(yp) = v.x;
+                        tmax = fmaxf(tmax, v.x);
+                        if (second)
                         {
-                            const float2 pw = *reinterpret_cast<const float2*>(sp);
-                            const float2 w = melW[k];
-                            fall.x = __fadd_rn(fall.x, __fmul_rn(pw.x, w.y));
-                            fall.y = __fadd_rn(fall.y, __fmul_rn(pw.y, w.y));
-                            rise.x = __fadd_rn(rise.x, __fmul_rn(pw.x, w.x));
-                            rise.y = __fadd_rn(rise.y, __fmul_rn(pw.y, w.x));
+                            *RPPB_WR(yp + 1) = v.y;
+                            tmax = fmaxf(tmax, v.y);
                         }
-                        if (i > m0)
-                        {
-                            *RPPB_WR(yp) = fall.x;
-                            tmax = fmaxf(tmax, fall.x);
-                            if (second)
-                            {
-                                *RPPB_WR(yp + 1) = fall.y;
-                                tmax = fmaxf(tmax, fall.y);
-                            }
-                            yp += hs;
-                        }
-                        fall = rise;
-                    }
+                        yp += hs;
+                    });
+                }
+                if constexpr (kPairs)
+                {
+                    // (the first tile's barriers come after the previous item's maxima have been read)
+                    tmax = warp_max(tmax);
+                    if ((tid & 31) == 0) s_warpMax[tid >> 5] = t == 0 ? tmax : fmaxf(s_warpMax[tid >> 5], tmax);
                 }
             }
-            tmax = warp_max(tmax);
-            if ((threadIdx.x & 31) == 0) s_warpMax[threadIdx.x >> 5] = tmax;
+            if constexpr (!kPairs)
+            {
+                tmax = warp_max(tmax);
+                if ((threadIdx.x & 31) == 0) s_warpMax[threadIdx.x >> 5] = tmax;
+            }
         }
         else
         {
@@ -200,6 +237,8 @@ __global__ void __launch_bounds__(kFusedThreads, (NFFT <= 512 ? 3 : 2)) frontend
                 s_ok = spins <= limit;
             }
             __syncthreads();
+            if constexpr (kPairs)
+                if (s_it[cur ^ 1].kind == 0) issue(s_it[cur ^ 1], s_it[cur ^ 1].f0);
             if (s_ok)
             {
                 float ref = a.refMag;
@@ -212,10 +251,11 @@ __global__ void __launch_bounds__(kFusedThreads, (NFFT <= 512 ? 3 : 2)) frontend
                 const int fd = threadIdx.x & (a.dbFrames - 1);   // dbFrames: power of two <= threads
                 const int gd = threadIdx.x / a.dbFrames;
                 const int kDbGroups = kFusedThreads / a.dbFrames;
-                if (fd < it.Tv)
-                {
+                auto convert = [&](auto normal) {
                     // 16 rows per step: the loads (mostly L2 hits) are in flight together (8: 1 % slower)
+                    constexpr bool kNormal = decltype(normal)::value;
                     constexpr int kRows = 16;
+                    const uint32_t hs = it.hs;
                     const size_t step = size_t(kDbGroups) * hs;
                     float* p = it.y + size_t(gd) * hs + fd;
                     int m = gd;
@@ -226,18 +266,15 @@ __global__ void __launch_bounds__(kFusedThreads, (NFFT <= 512 ? 3 : 2)) frontend
                         for (int r = 0; r < kRows; ++r) v[r] = __ldcg(RPPB_RD(p + r * step));
 #pragma unroll
                         for (int r = 0; r < kRows; ++r)
-                        {
-                            float t = __fmul_rn(v[r], inv);
-                            t = a.minRatio < t ? t : a.minRatio;
-                            *RPPB_WR(p + r * step) = __fmul_rn(a.multiplier, __log2f(t));
-                        }
+                            *RPPB_WR(p + r * step) = decibel<kNormal>(v[r], inv, a.minRatio, a.multiplier);
                     }
                     for (; m < nmel; m += kDbGroups, p += step)
-                    {
-                        float t = __fmul_rn(__ldcg(RPPB_RD(p)), inv);
-                        t = a.minRatio < t ? t : a.minRatio;
-                        *RPPB_WR(p) = __fmul_rn(a.multiplier, __log2f(t));
-                    }
+                        *RPPB_WR(p) = decibel<kNormal>(__ldcg(RPPB_RD(p)), inv, a.minRatio, a.multiplier);
+                };
+                if (fd < it.Tv)
+                {
+                    if (kPairs && a.minRatio >= kMinNormal) convert(std::true_type{});
+                    else convert(std::false_type{});
                 }
             }
         }
@@ -258,7 +295,7 @@ __global__ void __launch_bounds__(kFusedThreads, (NFFT <= 512 ? 3 : 2)) frontend
             prefetch_span(nx);
             s_it[cur] = nx;
         }
-        else if (threadIdx.x == 32 && it.kind == 0)
+        else if (threadIdx.x == 32 && kind == 0)
         {
             // the barrier orders every thread's mel stores before this thread's release, which
             // orders them (and the maximum) before the count
@@ -274,6 +311,7 @@ __global__ void __launch_bounds__(kFusedThreads, (NFFT <= 512 ? 3 : 2)) frontend
 template <int NFFT, int TFX>
 void launch_fused(Handle& h, const FrontendArgs& a, void* scratch)
 {
+    constexpr bool kPairs = PairPlan<NFFT>::use;
     using S = StftShape<NFFT, kFusedThreads, TFX>;
     const int nslots = a.n + a.lookahead;
     Carver cv(scratch);
@@ -281,12 +319,12 @@ void launch_fused(Handle& h, const FrontendArgs& a, void* scratch)
     unsigned long long* counter = cv.take<unsigned long long>(1);
     int* done = cv.take<int>(a.n);
     unsigned* maxKey = cv.take<unsigned>(a.n);
-    const FusedLayout<NFFT, TFX> lay(a.mel.numFilter, a.W, a.hop);
+    const FusedLayout<NFFT, TFX, kPairs> lay(a.mel.numFilter, a.W, a.hop);
     if (lay.total > 227 * 1024) fail(RPP_ERROR_OUT_OF_BOUND_SHARED_MEMORY_SIZE, "numFilter too large for the fused tile");
     const float2* tw = spectrogram_twiddles(h, NFFT);
     // the mel tables, built once per handle, mel parameters and tile (not while the stream is being
     // captured: then each CTA builds them)
-    uint4* melTables = fused_mel_table_cache<NFFT, TFX>(h, a);
+    uint4* melTables = fused_mel_table_cache<NFFT, TFX, kPairs>(h, a);
     // the prefix kernel also zeroes the queue counter, the tile counts and the maxima
     const size_t clear = reinterpret_cast<char*>(maxKey + a.n) - reinterpret_cast<char*>(counter);
     launch_ragged_prefix(SlotCount<S::TF>{a, a.n, a.lookahead}, nslots, prefix, h.stream(),

@@ -15,9 +15,11 @@
 
 #include "common.cuh"
 #include "handle.hpp"
+#include "mel_sweep.cuh"
 #include "mel_tables.cuh"
 #include "ops.hpp"
 #include "stft.cuh"
+#include "stft_pair.cuh"
 
 namespace rppb {
 
@@ -120,29 +122,30 @@ __device__ Item decode_item(const FrontendArgs& a, const SlotCount<TF>& cnt, con
     return it;
 }
 
-// Shared memory plan (bytes), computed identically on host and device.
-template <int NFFT, int TF>
+// Shared memory plan (bytes), computed identically on host and device.  kPairs: the sizes of stft_pair.cuh, where
+// the power tile takes the exchange slots' place.
+template <int NFFT, int TF, bool kPairs = false>
 struct FusedLayout
 {
     using S = StftShape<NFFT, kFusedThreads, TF>;
-    size_t tw, tw1, win, span, work, melW, melIv, melGrp, total;
+    static constexpr int kGroups = 2 * kFusedThreads / TF;   // mel thread groups: TF / 2 frame pairs each
+    // the parts that every thread addresses lie at constant offsets (no registers hold their addresses)
+    static constexpr size_t tw = 0, tw1 = tw + S::tw_bytes, win = tw1 + S::tw1_bytes, work = win + size_t(NFFT) * 4;
+    static constexpr size_t tileBytes = kPairs ? PairShape<NFFT>::slot_bytes : S::fft_bytes + S::out_bytes;
+    static constexpr size_t span = (work + tileBytes + 15) & ~size_t(15);
+    size_t cum, melW, melIv, melGrp, total;
     __host__ __device__ FusedLayout(int numFilter, int W, int hop)
     {
         const int bins = S::BINS;
-        tw = 0;
-        tw1 = tw + S::tw_bytes;
-        win = tw1 + S::tw1_bytes;
-        span = win + size_t(NFFT) * 4;
-        work = span + S::span_bytes(W, hop);
-        // the FFT slots + power tile, or (before the loop) the mel table build
-        size_t fftOut = S::fft_bytes + S::out_bytes;
+        // the FFT slots + power tile, then the span, or (before the loop) the mel table build
         size_t tables = 2 * size_t(numFilter + 2) * 4 + size_t(numFilter) * 4 + 2 * size_t(numFilter + 1) * 8 +
                         size_t(bins) * 4 + 64;
-        size_t workBytes = (fftOut > tables ? fftOut : tables);
-        melW = (work + workBytes + 15) & ~size_t(15);
+        cum = work + ((tables + 15) & ~size_t(15));
+        const size_t buildEnd = cum + size_t(numFilter + 1) * 4, tileEnd = span + S::span_bytes(W, hop);
+        melW = ((tileEnd > buildEnd ? tileEnd : buildEnd) + 15) & ~size_t(15);
         melIv = (melW + size_t(bins) * 8 + 15) & ~size_t(15);
         melGrp = (melIv + size_t(numFilter + 1) * 8 + 15) & ~size_t(15);
-        total = (melGrp + size_t(2 * kFusedThreads / TF + 1) * 4 + 15) & ~size_t(15);
+        total = (melGrp + size_t(kGroups + 1) * 4 + 15) & ~size_t(15);
     }
 };
 
@@ -151,15 +154,13 @@ struct FusedLayout
 // mel points i and i + 1) weighs (1 - wd_k) * norm_i into filter i and wd_k * norm_(i-1) into filter
 // i - 1, so filter m sums interval m's bins, then interval m + 1's, in ascending bin order -- the order
 // and the weights of the mel_filter_bank kernel.
-template <int NFFT, int TFX>
+template <int NFFT, int TFX, bool kPairs>
 __device__ __forceinline__ void build_fused_mel(const FrontendArgs& a, unsigned char* smem,
-                                                const FusedLayout<NFFT, TFX>& lay)
+                                                const FusedLayout<NFFT, TFX, kPairs>& lay)
 {
-    using S = StftShape<NFFT, kFusedThreads, TFX>;
-    constexpr int TF = S::TF, BINS = S::BINS;
-    constexpr int kGroups = 2 * kFusedThreads / TF;   // mel thread groups: TF / 2 frame pairs each
+    constexpr int BINS = NFFT / 2 + 1;
+    constexpr int kGroups = FusedLayout<NFFT, TFX, kPairs>::kGroups;
     const int nmel = a.mel.numFilter;
-    float* s_out = reinterpret_cast<float*>(smem + lay.work + S::fft_bytes);
     float2* melW = reinterpret_cast<float2*>(smem + lay.melW);   // bin k: (weight into filter i, into filter i - 1)
     int2* melIv = reinterpret_cast<int2*>(smem + lay.melIv);     // interval i: bins [x, y)
     int* melGrp = reinterpret_cast<int*>(smem + lay.melGrp);     // thread group g: filters [g], [g + 1])
@@ -193,9 +194,9 @@ __device__ __forceinline__ void build_fused_mel(const FrontendArgs& a, unsigned 
     }
     // group g emits filters [melGrp[g], melGrp[g + 1]) and sweeps their intervals; the groups'
     // shares of (bins + 2) per interval are balanced.  cum[i] = cost of intervals 0..i (an
-    // inclusive scan by warp 0, in the power tile's space, which is free until the first FFT);
+    // inclusive scan by warp 0, in the work region, which is free until the first FFT);
     // boundary g is 1 + the first filter m whose intervals 0..m+1 reach g / kGroups of the total.
-    int* cum = reinterpret_cast<int*>(s_out);
+    int* cum = reinterpret_cast<int*>(smem + lay.cum);
     for (int i = threadIdx.x; i <= nmel; i += kFusedThreads)
         cum[i] = (v.last[i] > v.first[i] ? v.last[i] - v.first[i] : 0) + 2;
     __syncthreads();
@@ -240,25 +241,25 @@ __device__ __forceinline__ void build_fused_mel(const FrontendArgs& a, unsigned 
 // Builds the fused kernel's mel tables once, with one CTA, into `out`: the bytes [melW, total) of its
 // shared-memory layout (melW, melIv, melGrp), which every launch with the same mel parameters and tile
 // copies instead of building them in each CTA.
-template <int NFFT, int TFX>
+template <int NFFT, int TFX, bool kPairs = false>
 __global__ void __launch_bounds__(kFusedThreads) fused_mel_tables_kernel(FrontendArgs a, uint4* __restrict__ out)
 {
     extern __shared__ __align__(16) unsigned char smem[];
-    const FusedLayout<NFFT, TFX> lay(a.mel.numFilter, a.W, a.hop);
-    build_fused_mel<NFFT, TFX>(a, smem, lay);
+    const FusedLayout<NFFT, TFX, kPairs> lay(a.mel.numFilter, a.W, a.hop);
+    build_fused_mel<NFFT, TFX, kPairs>(a, smem, lay);
     const uint4* src = reinterpret_cast<const uint4*>(smem + lay.melW);
     for (int i = threadIdx.x; i < int((lay.total - lay.melW) / 16); i += kFusedThreads) *RPPB_WR(out + i) = src[i];
 }
 
-// The fused kernels' mel tables (the bytes [melW, total) of FusedLayout<NFFT, TFX>), built once per
+// The fused kernels' mel tables (the bytes [melW, total) of FusedLayout), built once per
 // handle, mel parameters and tile by a one-CTA kernel on the handle stream and cached; nullptr while
 // the stream is being captured with parameters the handle has not cached (nothing is allocated during
 // capture).  Launched before the prefix kernel: the fused kernels read the tables before their
 // grid-dependency wait, which orders them only after the kernel just before them.
-template <int NFFT, int TFX>
+template <int NFFT, int TFX, bool kPairs = false>
 uint4* fused_mel_table_cache(Handle& h, const FrontendArgs& a)
 {
-    const FusedLayout<NFFT, TFX> lay(a.mel.numFilter, a.W, a.hop);
+    const FusedLayout<NFFT, TFX, kPairs> lay(a.mel.numFilter, a.W, a.hop);
     auto bits = [](float v) {
         uint32_t u;
         std::memcpy(&u, &v, sizeof u);
@@ -272,9 +273,9 @@ uint4* fused_mel_table_cache(Handle& h, const FrontendArgs& a)
     uint4* melTables = static_cast<uint4*>(h.device_table(key, lay.total - lay.melW, &fresh));
     if (fresh)
     {
-        const void* tk = reinterpret_cast<const void*>(fused_mel_tables_kernel<NFFT, TFX>);
+        const void* tk = reinterpret_cast<const void*>(fused_mel_tables_kernel<NFFT, TFX, kPairs>);
         persistent_grid(h, tk, kFusedThreads, lay.total);   // sets the kernel's shared-memory opt-in
-        fused_mel_tables_kernel<NFFT, TFX><<<1, kFusedThreads, lay.total, h.stream()>>>(a, melTables);
+        fused_mel_tables_kernel<NFFT, TFX, kPairs><<<1, kFusedThreads, lay.total, h.stream()>>>(a, melTables);
         count_launch();
         check_cuda(cudaGetLastError(), "fused_mel_tables_kernel");
     }

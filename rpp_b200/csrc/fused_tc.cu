@@ -459,39 +459,20 @@ __global__ void __launch_bounds__(kFusedThreads, 2)
                 __syncthreads();
                 if (fcol < Tv)
                 {
-                    // the FP32 kernel's mel sweep over the power tile (see fused.cu)
+                    // the FP32 kernel's mel sweep over the power tile
                     const bool second = fcol + 1 < Tv;
                     const int m0 = melGrp[g], m1 = melGrp[g + 1];
                     float* yp = it.y + size_t(f0 - it.f0) + size_t(m0) * hs + fcol;
-                    float2 fall = make_float2(0.f, 0.f);
-                    for (int i = m0; i <= m1; ++i)
-                    {
-                        const int2 iv = melIv[i];
-                        const float* sp = s_out + iv.x * LD + fcol;
-                        float2 rise = make_float2(0.f, 0.f);
-#pragma unroll 1
-                        for (int k = iv.x; k < iv.y; ++k, sp += LD)
+                    mel_sweep<LD>(s_out + fcol, melW, melIv, m0, m1, [&](float2 v) {
+                        *RPPB_WR(yp) = v.x;
+                        tmax = fmaxf(tmax, v.x);
+                        if (second)
                         {
-                            const float2 pw = *reinterpret_cast<const float2*>(sp);
-                            const float2 w = melW[k];
-                            fall.x = __fadd_rn(fall.x, __fmul_rn(pw.x, w.y));
-                            fall.y = __fadd_rn(fall.y, __fmul_rn(pw.y, w.y));
-                            rise.x = __fadd_rn(rise.x, __fmul_rn(pw.x, w.x));
-                            rise.y = __fadd_rn(rise.y, __fmul_rn(pw.y, w.x));
+                            *RPPB_WR(yp + 1) = v.y;
+                            tmax = fmaxf(tmax, v.y);
                         }
-                        if (i > m0)
-                        {
-                            *RPPB_WR(yp) = fall.x;
-                            tmax = fmaxf(tmax, fall.x);
-                            if (second)
-                            {
-                                *RPPB_WR(yp + 1) = fall.y;
-                                tmax = fmaxf(tmax, fall.y);
-                            }
-                            yp += hs;
-                        }
-                        fall = rise;
-                    }
+                        yp += hs;
+                    });
                 }
             }
             if (abort) break;

@@ -24,6 +24,7 @@
 #include "common.cuh"
 #include "ops.hpp"
 #include "stft.cuh"
+#include "stft_pair.cuh"
 
 namespace rppb {
 namespace {
@@ -122,6 +123,115 @@ __global__ void __launch_bounds__(kThreads, (NFFT <= 512 ? 3 : 2)) spectrogram_f
     }
 }
 
+// The same for the sizes of stft_pair.cuh.
+template <int NFFT>
+struct PairLayout
+{
+    using P = PairShape<NFFT>;
+    using S = StftShape<NFFT, P::THREADS, P::TF>;
+    size_t tw, tw1, win, span, slots, bytes;
+    __host__ __device__ PairLayout(int W, int hop)
+    {
+        tw = 0;
+        tw1 = tw + S::tw_bytes;
+        win = tw1 + S::tw1_bytes;
+        span = win + size_t(NFFT) * 4;
+        slots = span + S::span_bytes(W, hop);
+        bytes = slots + P::slot_bytes;
+    }
+};
+
+template <int NFFT>
+__global__ void __launch_bounds__(PairShape<NFFT>::THREADS, 4)
+    spectrogram_pair_kernel(SpectrogramArgs a, const float2* __restrict__ twiddle, const long long* __restrict__ prefix)
+{
+    using P = PairShape<NFFT>;
+    constexpr int TF = P::TF, BINS = P::BINS, THREADS = P::THREADS;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const PairLayout<NFFT> lay(a.windowLength, a.windowStep);
+    float2* s_tw = reinterpret_cast<float2*>(smem + lay.tw);
+    float2* s_tw1 = reinterpret_cast<float2*>(smem + lay.tw1);
+    float* s_win = reinterpret_cast<float*>(smem + lay.win);
+    float* s_span = reinterpret_cast<float*>(smem + lay.span);
+    float* s_slots = reinterpret_cast<float*>(smem + lay.slots);
+
+    const int W = a.windowLength, hop = a.windowStep;
+    stft_pair_tables<NFFT>(twiddle, a.window, W, s_tw, s_tw1, s_win, s_span);
+    const int centerOffset = a.center ? W / 2 : 0;
+    grid_dependency_wait();   // the prefix
+    prefix = dependency_result(prefix);
+    // a CTA takes consecutive tiles, so it finds its sample once and steps from there, and neighbouring tiles'
+    // partial output lines come from the same SM
+    const long long total = prefix[a.n];
+    const long long w0 = total * blockIdx.x / gridDim.x, w1 = total * (blockIdx.x + 1) / gridDim.x;
+    if (w0 >= w1) return;
+    int b = ragged_find(prefix, a.n, w0);
+    int f0 = int(w0 - *RPPB_RD(prefix + b)) * TF;
+    auto length = [&](int s) { return *RPPB_RD(a.len + s); };
+    auto frames = [&](int len) { return min(num_windows(len, W, hop, a.center), a.maxFrames); };
+    int L = length(b), F = frames(L);
+    const float* x = a.src + size_t(b) * a.srcStride;
+    bool issued = span_issue<NFFT, false>(x, L, f0, F, W, hop, centerOffset, s_span);
+    for (long long w = w0; w < w1; ++w)
+    {
+        span_arrive<NFFT>(issued, PlainSource{x, L, a.reflect}, f0, F, W, hop, centerOffset, s_span);
+        float2 z[P::R];
+        pair_gather<NFFT>(z, W, hop, s_win, s_span);
+        __syncthreads();   // the span buffer is free
+        // the next tile's samples travel from here on
+        int nb = b, nf0 = f0 + TF, nL = L, nF = F;
+        const float* nx = x;
+        issued = false;
+        if (w + 1 < w1)
+        {
+            while (nf0 >= nF)   // the next sample that has frames
+            {
+                nL = length(++nb);
+                nF = frames(nL);
+                nf0 = 0;
+                nx = a.src + size_t(nb) * a.srcStride;
+            }
+            issued = span_issue<NFFT, false>(nx, nL, nf0, nF, W, hop, centerOffset, s_span);
+        }
+        pair_transform<NFFT>(z, a.power, s_tw, s_tw1, s_slots);
+        __syncthreads();
+        const int Tv = min(TF, F - f0);
+        float* y = a.dst + size_t(b) * a.dstNStride;
+        if (a.nft)
+        {
+            // thread -> (frame f, bins k, k + THREADS / TF, ...): a warp writes TF consecutive frames of a bin
+            // (whole 16-byte pieces, with a tile's last frames carried into the next tile's first piece, cost
+            // more than they gave: 434 -> 462 us for the four plain calls on 256 clips)
+            constexpr int KS = THREADS / TF;
+            const int f = threadIdx.x % TF;
+            int k = threadIdx.x / TF;
+            if (f < Tv)
+            {
+                const float* sp = s_slots + (f >> 1) * P::PAIR_FLOATS + (f & 1) + 2 * k;
+                float* yp = y + size_t(k) * a.dstHStride + f0 + f;
+                const size_t ystep = size_t(KS) * a.dstHStride;
+#pragma unroll 8
+                for (; k < BINS; k += KS, sp += 2 * KS, yp += ystep) *RPPB_WR(yp) = *sp;
+            }
+        }
+        else
+        {
+            // thread -> consecutive bins of a pair's two frames
+            for (int idx = threadIdx.x; idx < BINS * P::PAIRS; idx += THREADS)
+            {
+                const int g = idx / BINS, k = idx % BINS;
+                if (2 * g >= Tv) break;
+                const float2 v = *reinterpret_cast<const float2*>(s_slots + g * P::PAIR_FLOATS + 2 * k);
+                float* yp = y + (size_t(f0 + 2 * g) * a.dstHStride + k);
+                *RPPB_WR(yp) = v.x;
+                if (2 * g + 1 < Tv) *RPPB_WR(yp + a.dstHStride) = v.y;
+            }
+        }
+        // the barriers of the next tile's staging precede its transforms' writes to the slots
+        b = nb, f0 = nf0, L = nL, F = nF, x = nx;
+    }
+}
+
 // Direct DFT for any nfft: one unit per (sample, frame).
 struct FrameCount
 {
@@ -199,6 +309,20 @@ void launch_fft(Handle& h, long long* prefix, const SpectrogramArgs& a, const fl
     check_cuda(cudaGetLastError(), "spectrogram_fft_kernel");
 }
 
+template <int NFFT>
+void launch_fft_pair(Handle& h, long long* prefix, const SpectrogramArgs& a, const float2* tw)
+{
+    using P = PairShape<NFFT>;
+    launch_ragged_prefix(SpecCount{a.len, a.windowLength, a.windowStep, a.maxFrames, P::TF, a.center}, a.n, prefix,
+                         h.stream());
+    const size_t smem = PairLayout<NFFT>(a.windowLength, a.windowStep).bytes;
+    if (smem > 227 * 1024) fail(RPP_ERROR_OUT_OF_BOUND_SHARED_MEMORY_SIZE, "window/hop too large for the frame tile");
+    const int grid = persistent_grid(h, reinterpret_cast<const void*>(spectrogram_pair_kernel<NFFT>), P::THREADS, smem);
+    launch_dependent(spectrogram_pair_kernel<NFFT>, dim3(grid), dim3(P::THREADS), smem, h.stream(),
+                     "spectrogram_pair_kernel", a, tw, static_cast<const long long*>(prefix));
+    count_launch();
+}
+
 void build_twiddle(float* out, size_t count, const void* ctx)
 {
     const int N = *static_cast<const int*>(ctx);
@@ -226,9 +350,9 @@ void launch_spectrogram(Handle& h, void* scratch, const SpectrogramArgs& a)
     const float2* tw = spectrogram_twiddles(h, a.nfft);
     switch (a.nfft)
     {
-        case 128: launch_fft<128>(h, prefix, a, tw); return;
+        case 128: launch_fft_pair<128>(h, prefix, a, tw); return;
         case 256: launch_fft<256>(h, prefix, a, tw); return;
-        case 512: launch_fft<512>(h, prefix, a, tw); return;
+        case 512: launch_fft_pair<512>(h, prefix, a, tw); return;
         case 1024: launch_fft<1024>(h, prefix, a, tw); return;
         case 2048: launch_fft<2048>(h, prefix, a, tw); return;
         default: break;

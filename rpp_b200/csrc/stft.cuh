@@ -60,10 +60,14 @@ struct StftShape
     static_assert(R1 % G == 0, "stage 2 assigns R1 / G rows per thread");
     // The window starts at offset (nfft - W) / 2 of the nfft buffer (0 when W >= nfft).
     __host__ __device__ static int window_offset(int W) { return W < NFFT ? (NFFT - W) / 2 : 0; }
-    // Span buffer: span_pad zero floats (>= the window offset, a multiple of 4), the tile's
+    // Span buffer: span_pad zero floats (a multiple of 4, at least the window offset; one more for the sizes of
+    // stft_pair.cuh, which keep the sample before the span there), the tile's
     // (TF - 1) * hop + W staged samples, then up to nfft - offset - W more zeros, so every frame
     // reads a full nfft-sample buffer without bounds checks (the window is 0 outside [0, W)).
-    __host__ __device__ static int span_pad(int W) { return (window_offset(W) + 3) & ~3; }
+    __host__ __device__ static int span_pad(int W)
+    {
+        return (window_offset(W) + (NFFT == 128 || NFFT == 512 ? 4 : 3)) & ~3;
+    }
     __host__ __device__ static int span_tail(int W)
     {
         const int t = NFFT - window_offset(W) - W;
