@@ -37,7 +37,8 @@ __global__ void __launch_bounds__(kThreads) down_mixing_kernel(const float* __re
                                                                const long long* __restrict__ prefix, int n)
 {
     __shared__ long long s_prefix[kPrefixCache];
-    prefix = cache_prefix(prefix, n, s_prefix);
+    grid_dependency_wait();
+    prefix = cache_prefix(dependency_result(prefix), n, s_prefix);
     const long long total = prefix[n];
     for (long long w = blockIdx.x; w < total; w += gridDim.x)
     {
@@ -72,9 +73,9 @@ void launch_down_mixing(Handle& h, void* scratch, const float* src, uint32_t src
     long long* prefix = static_cast<long long*>(scratch);
     launch_ragged_prefix(DownmixCount{dims}, n, prefix, h.stream());
     int grid = persistent_grid(h, reinterpret_cast<const void*>(down_mixing_kernel), kThreads, 0);
-    down_mixing_kernel<<<grid, kThreads, 0, h.stream()>>>(src, srcStride, dst, dstStride, dims, normalize, prefix, n);
+    launch_dependent(down_mixing_kernel, dim3(grid), dim3(kThreads), 0, h.stream(), "down_mixing_kernel", src, srcStride,
+                     dst, dstStride, dims, normalize, static_cast<const long long*>(prefix), n);
     count_launch();
-    check_cuda(cudaGetLastError(), "down_mixing_kernel");
 }
 
 }  // namespace rppb

@@ -16,6 +16,7 @@
 #include <cfloat>
 
 #include "common.cuh"
+#include "mel_sweep.cuh"
 #include "mel_tables.cuh"
 #include "ops.hpp"
 
@@ -147,8 +148,16 @@ __global__ void __launch_bounds__(kThreads) mel_kernel(MelArgs a, float maxFreq,
     const MelParams mp{a.minFreq, maxFreq, a.sampleRate, a.htk, a.numFilter, a.normalize};
     if (threadIdx.x == 0) range[2] = -1;
     __syncthreads();
+    // the tables of the first sample's bins, as a rule everyone's, while the prefix kernel runs
+    const int firstBins = *RPPB_RD(a.dims);
+    if (firstBins >= 2 && firstBins <= maxBins)
+    {
+        build_mel_tables(T, mp, (firstBins - 1) * 2);
+        build_sweep(T, a.numFilter, a.normalize, weights, intervals, groups, reinterpret_cast<int*>(smem + lay.cum));
+    }
     __shared__ long long s_prefix[kPrefixCache];
-    prefix = cache_prefix(prefix, a.n, s_prefix);
+    grid_dependency_wait();
+    prefix = cache_prefix(dependency_result(prefix), a.n, s_prefix);
     const long long total = prefix[a.n];
     const int t = 2 * (threadIdx.x % kPairs);   // first of this thread's two frames
     const int g = threadIdx.x / kPairs;
@@ -203,30 +212,12 @@ __global__ void __launch_bounds__(kThreads) mel_kernel(MelArgs a, float maxFreq,
             const bool live0 = ok && col < frames, live1 = ok && col + 1 < frames, has1 = col + 1 < zc;
             const int m0 = ok ? groups[g] : 0, m1 = ok ? groups[g + 1] : 0;
             float* yp = a.dst + size_t(b) * a.dstNStride + size_t(m0) * a.dstHStride + col;
-            float2 fall = make_float2(0.f, 0.f);   // filter i - 1: rising sum, then falling terms
-            for (int i = m0; i <= m1 && ok; ++i)
-            {
-                const int2 iv = intervals[i];
-                const float* sp = s_spec + (iv.x - k0) * kLd + t;
-                float2 rise = make_float2(0.f, 0.f);   // filter i
-#pragma unroll 1
-                for (int k = iv.x; k < iv.y; ++k, sp += kLd)
-                {
-                    const float2 pw = *reinterpret_cast<const float2*>(sp);
-                    const float2 w = weights[k];
-                    fall.x = __fadd_rn(fall.x, __fmul_rn(pw.x, w.y));
-                    fall.y = __fadd_rn(fall.y, __fmul_rn(pw.y, w.y));
-                    rise.x = __fadd_rn(rise.x, __fmul_rn(pw.x, w.x));
-                    rise.y = __fadd_rn(rise.y, __fmul_rn(pw.y, w.x));
-                }
-                if (i > m0)
-                {
-                    *RPPB_WR(yp) = live0 ? fall.x : 0.0f;
-                    if (has1) *RPPB_WR(yp + 1) = live1 ? fall.y : 0.0f;
+            if (ok)
+                mel_sweep<kLd>(s_spec - k0 * kLd + t, weights, intervals, m0, m1, [&](float2 v) {
+                    *RPPB_WR(yp) = live0 ? v.x : 0.0f;
+                    if (has1) *RPPB_WR(yp + 1) = live1 ? v.y : 0.0f;
                     yp += a.dstHStride;
-                }
-                fall = rise;
-            }
+                });
             if (!ok)   // no tables for this sample: zeros, as the reference leaves its output
                 for (int m = g; m < a.numFilter; m += kGroups)
                 {
@@ -251,9 +242,9 @@ void launch_mel_filter_bank(Handle& h, void* scratch, const MelArgs& a)
     launch_ragged_prefix(MelCount{a.dims, a.dstHStride}, a.n, prefix, h.stream());
     const float maxFreq = (a.maxFreq == 0) ? a.sampleRate / 2 : a.maxFreq;
     int grid = persistent_grid(h, reinterpret_cast<const void*>(mel_kernel), kThreads, smem);
-    mel_kernel<<<grid, kThreads, smem, h.stream()>>>(a, maxFreq, maxBins, prefix);
+    launch_dependent(mel_kernel, dim3(grid), dim3(kThreads), smem, h.stream(), "mel_kernel", a, maxFreq, maxBins,
+                     static_cast<const long long*>(prefix));
     count_launch();
-    check_cuda(cudaGetLastError(), "mel_kernel");
 }
 
 }  // namespace rppb

@@ -37,7 +37,8 @@ __global__ void __launch_bounds__(kThreads) pre_emphasis_kernel(const float* __r
                                                                 int n)
 {
     __shared__ long long s_prefix[kPrefixCache];
-    prefix = cache_prefix(prefix, n, s_prefix);
+    grid_dependency_wait();
+    prefix = cache_prefix(dependency_result(prefix), n, s_prefix);
     const long long total = prefix[n];
     const int lane = threadIdx.x & 31;
     for (long long w = blockIdx.x; w < total; w += gridDim.x)
@@ -107,18 +108,19 @@ void launch_pre_emphasis(Handle& h, void* scratch, const float* src, uint32_t sr
     if (vec)
     {
         int grid = persistent_grid(h, reinterpret_cast<const void*>(pre_emphasis_kernel<true>), kThreads, 0);
-        pre_emphasis_kernel<true><<<grid, kThreads, 0, h.stream()>>>(src, srcStride, dst, dstStride, len, coeff,
-                                                                     border, srcElems, prefix, n);
+        launch_dependent(pre_emphasis_kernel<true>, dim3(grid), dim3(kThreads), 0, h.stream(), "pre_emphasis_kernel", src,
+                         srcStride, dst, dstStride, len, coeff, border, srcElems,
+                         static_cast<const long long*>(prefix), n);
         count_launch();
     }
     else
     {
         int grid = persistent_grid(h, reinterpret_cast<const void*>(pre_emphasis_kernel<false>), kThreads, 0);
-        pre_emphasis_kernel<false><<<grid, kThreads, 0, h.stream()>>>(src, srcStride, dst, dstStride, len, coeff,
-                                                                      border, srcElems, prefix, n);
+        launch_dependent(pre_emphasis_kernel<false>, dim3(grid), dim3(kThreads), 0, h.stream(), "pre_emphasis_kernel",
+                         src, srcStride, dst, dstStride, len, coeff, border, srcElems,
+                         static_cast<const long long*>(prefix), n);
         count_launch();
     }
-    check_cuda(cudaGetLastError(), "pre_emphasis_kernel");
 }
 
 }  // namespace rppb

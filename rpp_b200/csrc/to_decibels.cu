@@ -79,7 +79,8 @@ __global__ void __launch_bounds__(kThreads) decibel_max_kernel(const float* __re
 {
     __shared__ float warpMax[kThreads / 32];
     __shared__ long long s_prefix[kPrefixCache];
-    prefix = cache_prefix(prefix, n, s_prefix);
+    grid_dependency_wait();   // the prefix and the zeroed maxima
+    prefix = cache_prefix(dependency_result(prefix), n, s_prefix);
     const long long total = prefix[n];
     for (long long w = blockIdx.x; w < total; w += gridDim.x)
     {
@@ -132,7 +133,7 @@ __global__ void __launch_bounds__(kThreads) decibel_max_kernel(const float* __re
     }
 }
 
-template <bool kUseMax>
+template <bool kUseMax, bool kNormal>
 __global__ void __launch_bounds__(kThreads) decibel_kernel(const float* __restrict__ src, uint32_t srcNStride,
                                                            uint32_t srcHStride, float* __restrict__ dst,
                                                            uint32_t dstNStride, uint32_t dstHStride,
@@ -142,7 +143,9 @@ __global__ void __launch_bounds__(kThreads) decibel_kernel(const float* __restri
                                                            const long long* __restrict__ prefix, int n, bool vec)
 {
     __shared__ long long s_prefix[kPrefixCache];
-    prefix = cache_prefix(prefix, n, s_prefix);
+    grid_dependency_wait();   // the prefix, the maxima
+    maxKey = dependency_result(maxKey);
+    prefix = cache_prefix(dependency_result(prefix), n, s_prefix);
     const long long total = prefix[n];
     for (long long w = blockIdx.x; w < total; w += gridDim.x)
     {
@@ -156,11 +159,7 @@ __global__ void __launch_bounds__(kThreads) decibel_kernel(const float* __restri
             ref = k == 0u ? -FLT_MAX : fmaxf(-FLT_MAX, key_float(k));
         }
         const float inv = ref != 0.f ? __fdiv_rn(1.f, ref) : 1.0f;
-        auto db = [&](float x) {
-            float t = __fmul_rn(x, inv);
-            t = minRatio < t ? t : minRatio;
-            return __fmul_rn(multiplier, __log2f(t));
-        };
+        auto db = [&](float x) { return decibel<kNormal>(x, inv, minRatio, multiplier); };
         // in-place calls alias src and dst: every element is loaded before its own store.  A lane
         // loads 4 column steps (16 values) before converting and storing them, so the loads overlap.
         const float* xb = src + size_t(b) * srcNStride + size_t(s.row) * srcHStride + s.col0;
@@ -211,6 +210,12 @@ __global__ void __launch_bounds__(kThreads) decibel_kernel(const float* __restri
     }
 }
 
+template <bool kUseMax>
+auto pick_decibel_kernel(float minRatio)
+{
+    return minRatio >= kMinNormal ? decibel_kernel<kUseMax, true> : decibel_kernel<kUseMax, false>;
+}
+
 }  // namespace
 
 void launch_to_decibels(Handle& h, void* scratch, const DecibelArgs& a)
@@ -219,6 +224,7 @@ void launch_to_decibels(Handle& h, void* scratch, const DecibelArgs& a)
     Carver cv(scratch);
     long long* prefix = cv.take<long long>(a.n + 1);
     unsigned* maxKey = cv.take<unsigned>(a.n);
+    const long long* cprefix = prefix;
     const bool useMax = (a.referenceMagnitude == 0.f);
     // the maxima accumulate with atomicMax from zero keys: the prefix kernel zeroes them
     launch_ragged_prefix(DecibelCount{a.dims}, a.n, prefix, h.stream(), maxKey, useMax ? a.n : 0);
@@ -228,26 +234,25 @@ void launch_to_decibels(Handle& h, void* scratch, const DecibelArgs& a)
     if (useMax)
     {
         int grid = persistent_grid(h, reinterpret_cast<const void*>(decibel_max_kernel), kThreads, 0);
-        decibel_max_kernel<<<grid, kThreads, 0, h.stream()>>>(a.src, a.srcNStride, a.srcHStride, a.dims, maxKey,
-                                                              prefix, a.n, vecSrc);
+        launch_dependent(decibel_max_kernel, dim3(grid), dim3(kThreads), 0, h.stream(), "decibel_max_kernel", a.src,
+                         a.srcNStride, a.srcHStride, a.dims, maxKey, cprefix, a.n, vecSrc);
         count_launch();
-        check_cuda(cudaGetLastError(), "decibel_max_kernel");
-        grid = persistent_grid(h, reinterpret_cast<const void*>(decibel_kernel<true>), kThreads, 0);
-        decibel_kernel<true><<<grid, kThreads, 0, h.stream()>>>(a.src, a.srcNStride, a.srcHStride, a.dst, a.dstNStride,
-                                                                a.dstHStride, a.dims, maxKey, 0.f, a.minRatio,
-                                                                a.multiplier, prefix, a.n, vec);
+        const auto kernel = pick_decibel_kernel<true>(a.minRatio);
+        grid = persistent_grid(h, reinterpret_cast<const void*>(kernel), kThreads, 0);
+        launch_dependent(kernel, dim3(grid), dim3(kThreads), 0, h.stream(), "decibel_kernel", a.src, a.srcNStride,
+                         a.srcHStride, a.dst, a.dstNStride, a.dstHStride, a.dims, static_cast<const unsigned*>(maxKey),
+                         0.f, a.minRatio, a.multiplier, cprefix, a.n, vec);
         count_launch();
     }
     else
     {
-        int grid = persistent_grid(h, reinterpret_cast<const void*>(decibel_kernel<false>), kThreads, 0);
-        decibel_kernel<false><<<grid, kThreads, 0, h.stream()>>>(a.src, a.srcNStride, a.srcHStride, a.dst,
-                                                                 a.dstNStride, a.dstHStride, a.dims, nullptr,
-                                                                 a.referenceMagnitude, a.minRatio, a.multiplier,
-                                                                 prefix, a.n, vec);
+        const auto kernel = pick_decibel_kernel<false>(a.minRatio);
+        int grid = persistent_grid(h, reinterpret_cast<const void*>(kernel), kThreads, 0);
+        launch_dependent(kernel, dim3(grid), dim3(kThreads), 0, h.stream(), "decibel_kernel", a.src, a.srcNStride,
+                         a.srcHStride, a.dst, a.dstNStride, a.dstHStride, a.dims, static_cast<const unsigned*>(nullptr),
+                         a.referenceMagnitude, a.minRatio, a.multiplier, cprefix, a.n, vec);
         count_launch();
     }
-    check_cuda(cudaGetLastError(), "decibel_kernel");
 }
 
 }  // namespace rppb
@@ -292,9 +297,9 @@ cudaError_t static_setup(int device, StaticDevice*& out)
         if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess) return e;
         if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, decibel_max_kernel, kThreads, 0)) != cudaSuccess)
             return e;
-        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, decibel_kernel<true>, kThreads, 0)) != cudaSuccess)
+        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, decibel_kernel<true, true>, kThreads, 0)) != cudaSuccess)
             return e;
-        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, decibel_kernel<false>, kThreads, 0)) != cudaSuccess)
+        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, decibel_kernel<false, true>, kThreads, 0)) != cudaSuccess)
             return e;
         d.scratch = static_cast<unsigned char*>(p);
         d.gridMax = max(a, 1) * sms;
@@ -375,15 +380,14 @@ extern "C" SHARED_PUBLIC RppStatus rppt_to_decibels_gpu_static(RppPtr_t srcPtr, 
         decibel_max_kernel<<<sd->gridMax, kThreads, 0, s>>>(src, sN, sH, dims, maxKey, prefix, n, vecSrc);
         count_launch();
         if (cudaGetLastError() != cudaSuccess) return RPP_ERROR;
-        decibel_kernel<true><<<sd->gridTrue, kThreads, 0, s>>>(src, sN, sH, dst, dN, dH, dims, maxKey, 0.f, minRatio,
-                                                               multiplier, prefix, n, vec);
+        pick_decibel_kernel<true>(minRatio)<<<sd->gridTrue, kThreads, 0, s>>>(
+            src, sN, sH, dst, dN, dH, dims, maxKey, 0.f, minRatio, multiplier, prefix, n, vec);
         count_launch();
     }
     else
     {
-        decibel_kernel<false><<<sd->gridFalse, kThreads, 0, s>>>(src, sN, sH, dst, dN, dH, dims, nullptr,
-                                                                 referenceMagnitude, minRatio, multiplier, prefix, n,
-                                                                 vec);
+        pick_decibel_kernel<false>(minRatio)<<<sd->gridFalse, kThreads, 0, s>>>(
+            src, sN, sH, dst, dN, dH, dims, nullptr, referenceMagnitude, minRatio, multiplier, prefix, n, vec);
         count_launch();
     }
     return cudaGetLastError() == cudaSuccess ? RPP_SUCCESS : RPP_ERROR;
