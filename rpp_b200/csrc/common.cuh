@@ -144,12 +144,14 @@ __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepco
 
 // The pointer to something that the kernel waited for has written, to be taken after grid_dependency_wait():
 // through a const __restrict__ parameter the compiler may load before the wait (it takes the memory for
-// constant), through the returned pointer it cannot.
+// constant), through the returned pointer it cannot.  The address passes as a global one, so that accesses
+// through the result stay global, not generic.
 template <class T>
 __device__ __forceinline__ T* dependency_result(T* p)
 {
-    asm volatile("" : "+l"(p)::"memory");
-    return p;
+    size_t g = __cvta_generic_to_global(p);
+    asm volatile("" : "+l"(g)::"memory");
+    return static_cast<T*>(const_cast<void*>(static_cast<const void*>(__cvta_global_to_generic(g))));
 }
 
 // Launches `kernel` with programmatic stream serialization: it may start while the kernel before

@@ -128,10 +128,14 @@ __global__ void __launch_bounds__(kFusedThreads, (NFFT <= 512 ? 3 : 2)) frontend
     int cur = 0;
     if (threadIdx.x == 0)
     {
+        // the second claim waits until the first is decoded, so that every CTA has its first item before any has
+        // its second: claimed back to back, a small batch's items pair up in half of the CTAs (37 clips of 0.3 to 5 s:
+        // 52 us back to back, 43 us with the second after the first's return, 31 us after its decoding)
         const long long w0 = (long long)atomicAdd(RPPB_WR(workCounter), 1ull);
-        const long long w1 = (long long)atomicAdd(RPPB_WR(workCounter), 1ull);
-        wAfter = w1 < total - 2ll * gridDim.x ? (long long)atomicAdd(RPPB_WR(workCounter), 1ull) : -1ll;
         s_it[0] = decode_item<TF>(a, cnt, prefix, nslots, total, w0);
+        asm volatile("" ::: "memory");
+        const long long w1 = (long long)atomicAdd(RPPB_WR(workCounter + (w0 >> 63)), 1ull);   // (w0 >= 0)
+        wAfter = w1 < total - 2ll * gridDim.x ? (long long)atomicAdd(RPPB_WR(workCounter), 1ull) : -1ll;
         s_it[1] = decode_item<TF>(a, cnt, prefix, nslots, total, w1);
         prefetch_span(s_it[1]);
     }

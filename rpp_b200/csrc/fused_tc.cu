@@ -359,10 +359,12 @@ __global__ void __launch_bounds__(kFusedThreads, 2)
     int cur = 0;
     if (threadIdx.x == 0)
     {
+        // the second claim after the first item's decoding: every CTA has an item before any has two
         const long long w0 = (long long)atomicAdd(RPPB_WR(workCounter), 1ull);
-        const long long w1 = (long long)atomicAdd(RPPB_WR(workCounter), 1ull);
-        wAfter = w1 < total - 2ll * gridDim.x ? (long long)atomicAdd(RPPB_WR(workCounter), 1ull) : -1ll;
         s_it[0] = decode_item<TF>(a, cnt, prefix, nslots, total, w0);
+        asm volatile("" ::: "memory");
+        const long long w1 = (long long)atomicAdd(RPPB_WR(workCounter + (w0 >> 63)), 1ull);   // (w0 >= 0)
+        wAfter = w1 < total - 2ll * gridDim.x ? (long long)atomicAdd(RPPB_WR(workCounter), 1ull) : -1ll;
         s_it[1] = decode_item<TF>(a, cnt, prefix, nslots, total, w1);
         prefetch_span(s_it[1]);
     }
