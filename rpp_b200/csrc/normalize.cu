@@ -210,37 +210,58 @@ __global__ void __launch_bounds__(kThreads) normalize_kernel(NormalizeArgs a, co
     }
 }
 
-// The sum of a node of the halving tree whose elements one lane sums.
+// The sum of a node of the halving tree whose elements one lane sums (n <= 128).
 template <bool kSq>
 __device__ __forceinline__ float subtree_sum(const float* in, int n, float mean)
 {
-    auto run = [&](int i0, int i1) {
+    auto run = [&](const float* p, int m) {
         float t = 0.f;
-        for (int i = i0; i < i1; ++i)
+#pragma unroll 4
+        for (int i = 0; i < m; ++i)
         {
-            const float c = kSq ? __fsub_rn(in[i], mean) : in[i];
+            const float c = kSq ? __fsub_rn(p[i], mean) : p[i];
             t = __fadd_rn(t, kSq ? __fmul_rn(c, c) : c);
         }
         return t;
     };
-    if (n <= 32) return run(0, n);
-    if (n <= 64) return __fadd_rn(run(0, n >> 1), run(n >> 1, n));
-    return tree_sum<kSq>(in, 1, n, mean);
+    auto square = [&](float v) {
+        const float c = kSq ? __fsub_rn(v, mean) : v;
+        return kSq ? __fmul_rn(c, c) : c;
+    };
+    auto node = [&](const float* p, int m) {
+        if (m <= 32) return run(p, m);
+        // both halves at once: two chains in flight
+        const int h = m >> 1;
+        const float* q = p + h;
+        float t = 0.f, u = 0.f;
+#pragma unroll 4
+        for (int i = 0; i < h; ++i)
+        {
+            t = __fadd_rn(t, square(p[i]));
+            u = __fadd_rn(u, square(q[i]));
+        }
+        if (m & 1) u = __fadd_rn(u, square(q[h]));
+        return __fadd_rn(t, u);
+    };
+    return n <= 64 ? node(in, n) : __fadd_rn(node(in, n >> 1), node(in + (n >> 1), n - (n >> 1)));
 }
 
 // Rows of one warp each: statistics over the row and the normalized row, with the row's elements read once.
-// The row is staged in shared memory; the top `depth` levels of the halving tree are dealt to 2^depth lanes
-// (every node above them holds more than 32 elements, so it splits), which sum their subtrees and combine
-// them pairwise in tree order.  One read and one write per element: HBM-bound.  It replaces a statistics
-// pass with a lane per row (below 544 elements) or a warp per row, then a second pass over the rows:
-// per-filter normalization of 256 clips' decibels (128 x 101 to 1601) 209 + 103 us.
+// The row is staged in shared memory by asynchronous copies, all of them in flight at once, while the warp's next row
+// travels to L2; the top `depth` levels of the halving tree are dealt to 2^depth lanes (every node above them holds
+// more than 32 elements, so it splits), which sum their subtrees and combine them pairwise in tree order.  One read
+// and one write per element.  It replaces a statistics pass with a lane per row (below 544 elements) or a warp per
+// row, then a second pass over the rows: per-filter normalization of 256 clips' decibels (128 x 101 to 1601)
+// 209 + 103 us there, 80 us here (90 with 16 loads per lane at a time through registers).  Latency and instructions
+// bound it: rows skewed against bank conflicts cost more than they gave (96 against 87 us per call).
 __global__ void __launch_bounds__(kThreads) normalize_rows_kernel(NormalizeArgs a, int rowsPerSample, int stage)
 {
     extern __shared__ float s_rows[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float* row = s_rows + warp * stage;
     const long long rows = (long long)a.n * rowsPerSample;
-    for (long long u = blockIdx.x * (kThreads / 32) + warp; u < rows; u += (long long)gridDim.x * (kThreads / 32))
+    const long long step = (long long)gridDim.x * (kThreads / 32);
+    for (long long u = blockIdx.x * (kThreads / 32) + warp; u < rows; u += step)
     {
         const int b = int(u / rowsPerSample);
         const uint32_t r = uint32_t(u - (long long)b * rowsPerSample);
@@ -255,17 +276,17 @@ __global__ void __launch_bounds__(kThreads) normalize_rows_kernel(NormalizeArgs 
             n = s.count;
             const float* x = a.src + size_t(b) * a.srcStride0 + size_t(r) * a.srcStride1;
             __syncwarp();   // the previous row's reads are done
-            constexpr int kBatch = 16;
-            for (int i0 = lane; i0 < n; i0 += kBatch * 32)
+            for (int i = lane; i < n; i += 32) copy_async4(row + i, x + i);
+            // the warp's next row travels to L2 while this one is summed
+            if (lane == 0 && u + step < rows)
             {
-                float v[kBatch];
-#pragma unroll
-                for (int k = 0; k < kBatch; ++k)
-                    if (i0 + 32 * k < n) v[k] = __ldg(RPPB_RD(x + (i0 + 32 * k)));
-#pragma unroll
-                for (int k = 0; k < kBatch; ++k)
-                    if (i0 + 32 * k < n) row[i0 + 32 * k] = v[k];
+                const int bn = int((u + step) / rowsPerSample);
+                const uint32_t rn = uint32_t(u + step - (long long)bn * rowsPerSample);
+                const NormalizeSample sn = *RPPB_RD(a.samples + bn);
+                const float* xn = a.src + size_t(bn) * a.srcStride0 + size_t(rn) * a.srcStride1;
+                if (rn < uint32_t(sn.len0)) l2_prefetch(xn, xn + sn.count);
             }
+            copy_async_wait();
             __syncwarp();
             int depth = 0;
             while (depth < 5 && (n >> depth) > 32) ++depth;

@@ -54,19 +54,6 @@ struct PairShape
 // Pre-emphasis in the gather costs 2.5 times the operations of one pass over the span (hop 160 of 400), and neither
 // that pass's shared-memory round trip nor its two barriers.
 
-__device__ __forceinline__ void copy_async16(float* to, const float* from)
-{
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(uint32_t(__cvta_generic_to_shared(to))),
-                 "l"(RPPB_RD(reinterpret_cast<const float4*>(from)))
-                 : "memory");
-}
-__device__ __forceinline__ void copy_async4(float* to, const float* from)
-{
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(uint32_t(__cvta_generic_to_shared(to))),
-                 "l"(RPPB_RD(from))
-                 : "memory");
-}
-
 // Starts the copies of the span of frames f0 .. f0+TF-1 (those < F) and zeroes its tail.  False (and nothing
 // started) for a tile that reaches past the signal, or, kPreemph, before its second sample.  The sample before the
 // span goes into the last float of the pad (kPreemph).  The span buffer must be free.
