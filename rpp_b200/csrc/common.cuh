@@ -200,17 +200,17 @@ __device__ __forceinline__ void l2_prefetch(const float* begin, const float* end
 }
 
 // Asynchronous copies of 16 or 4 aligned bytes from global to shared memory (cp.async; the issuing thread waits for
-// its own with copy_async_wait).
-__device__ __forceinline__ void copy_async16(float* to, const float* from)
+// its own with copy_async_wait).  The caller passes its source through RPPB_RD.
+__device__ __forceinline__ void copy_async16(float* to, const float4* from)
 {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(uint32_t(__cvta_generic_to_shared(to))),
-                 "l"(RPPB_RD(reinterpret_cast<const float4*>(from)))
+                 "l"(from)
                  : "memory");
 }
 __device__ __forceinline__ void copy_async4(float* to, const float* from)
 {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(uint32_t(__cvta_generic_to_shared(to))),
-                 "l"(RPPB_RD(from))
+                 "l"(from)
                  : "memory");
 }
 __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }

@@ -252,7 +252,7 @@ __device__ __forceinline__ float subtree_sum(const float* in, int n, float mean)
 // more than 32 elements, so it splits), which sum their subtrees and combine them pairwise in tree order.  One read
 // and one write per element.  It replaces a statistics pass with a lane per row (below 544 elements) or a warp per
 // row, then a second pass over the rows: per-filter normalization of 256 clips' decibels (128 x 101 to 1601)
-// 209 + 103 us there, 80 us here (90 with 16 loads per lane at a time through registers).  Latency and instructions
+// 209 + 103 us there, 77 us here (90 with 16 loads per lane at a time through registers).  Latency and instructions
 // bound it: rows skewed against bank conflicts cost more than they gave (96 against 87 us per call).
 __global__ void __launch_bounds__(kThreads) normalize_rows_kernel(NormalizeArgs a, int rowsPerSample, int stage)
 {
@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(kThreads) normalize_rows_kernel(NormalizeArgs 
             n = s.count;
             const float* x = a.src + size_t(b) * a.srcStride0 + size_t(r) * a.srcStride1;
             __syncwarp();   // the previous row's reads are done
-            for (int i = lane; i < n; i += 32) copy_async4(row + i, x + i);
+            for (int i = lane; i < n; i += 32) copy_async4(row + i, RPPB_RD(x + i));
             // the warp's next row travels to L2 while this one is summed
             if (lane == 0 && u + step < rows)
             {

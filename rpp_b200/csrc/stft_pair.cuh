@@ -69,13 +69,14 @@ __device__ __forceinline__ bool span_issue(const float* __restrict__ x, int L, i
     float* to = s_span + S::span_pad(W);
     if ((reinterpret_cast<uintptr_t>(from) & 15) == 0)
     {
-        for (int i = 4 * threadIdx.x; i + 4 <= len; i += 4 * P::THREADS) copy_async16(to + i, from + i);
+        for (int i = 4 * threadIdx.x; i + 4 <= len; i += 4 * P::THREADS)
+            copy_async16(to + i, RPPB_RD(reinterpret_cast<const float4*>(from + i)));
         const int i = (len & ~3) + threadIdx.x;
-        if (i < len) copy_async4(to + i, from + i);
+        if (i < len) copy_async4(to + i, RPPB_RD(from + i));
     }
     else
-        for (int i = threadIdx.x; i < len; i += P::THREADS) copy_async4(to + i, from + i);
-    if (kPreemph && threadIdx.x == 0) copy_async4(to - 1, from - 1);
+        for (int i = threadIdx.x; i < len; i += P::THREADS) copy_async4(to + i, RPPB_RD(from + i));
+    if (kPreemph && threadIdx.x == 0) copy_async4(to - 1, RPPB_RD(from - 1));
     asm volatile("cp.async.commit_group;" ::: "memory");
     for (int i = threadIdx.x; i < S::span_tail(W); i += P::THREADS) to[len + i] = 0.f;
     return true;
