@@ -77,8 +77,9 @@ __global__ void __launch_bounds__(kFusedThreads, (NFFT <= 512 ? 3 : 2)) frontend
 
     // The per-CTA setup (tables below) runs in a loop whose trip count, always one, the compiler
     // cannot prove: the setup's registers are then allocated apart from the work loop's, which keeps
-    // the work loop free of spills at the 80-register cap (ptxas, nfft 512: 0 bytes of spill stores
-    // instead of 48; 263 -> 253 us on the 256-clip batch, bit-identical).
+    // the work loop nearly free of spills at the 80-register cap (ptxas, nfft 512: 8 bytes of spill
+    // stores; with the span staged through registers 0 instead of 48, 263 -> 253 us on the 256-clip
+    // batch, bit-identical).
     for (int setupPass = 0, setupPasses = 1 + (a.n < 0); setupPass < setupPasses; ++setupPass)
     {
         // the mel tables: copied from the handle's cache when the launch has them, else built here

@@ -10,7 +10,7 @@
 //   - the window is halved (exact), which takes the place of the unpack's factors of 1/2;
 //   - the next tile's samples are copied into the span buffer while this tile is transformed.
 // On 256 clips of 1 to 16 s (nfft 512) the spectrogram kernel takes 176 us instead of 221 (ncu) and the fused front
-// end, which keeps 80 registers and three CTAs (64 registers spill: 302 us), 253 us instead of 262.  The transform is
+// end, which keeps 80 registers and three CTAs (64 registers spill: 302 us), 251 us instead of 262.  The transform is
 // not what bounds the spectrogram: without it the kernel takes 167 us, without its stores 52.
 // Two frames per lane group in the halves of paired instructions (fewer instructions, 128 registers, 16 warps per
 // SM) took 202 and 281 us.
