@@ -14,17 +14,22 @@
 // first (last) candidate's interval meets the cutoff's.  Only then is that candidate's reset block
 // replayed, in exactly the reference's order (add the new square, store sum * (1/windowLength), subtract
 // the square leaving the window; explicit round-to-nearest intrinsics, no FMA), and, if its exact values
-// lie inside the cutoff's interval too, the blocks that may hold the maximum.  Begin and length are
-// therefore the host path's on every input.
-//   1. energy_kernel: FP64 energies of 64-sample chunks, one streaming pass over the signal (HBM-bound: 31 us
+// lie inside the cutoff's interval too, the blocks that may hold the maximum.  Clips that this does not settle have
+// every block replayed.  Begin and length are therefore the host path's on every input.
+//   1. energy_kernel: FP64 energies of 64-sample chunks, one streaming pass over the signal (HBM-bound: 30 us
 //      for 256 clips of 1 to 16 s, 4.6 TB/s);
 //   2. region_kernel: one CTA per sample: scan of the energies, cutoff interval, both ends, replays (15 to
-//      20 us without a replay, 73 us with one).
+//      20 us without a replay, about 50 us more for each one);
+//   3. exact_kernel: the reset blocks of the samples that are left, over the whole GPU (3 us with none).
 // A clip that ends in silence after sound within one reset block needs a replay as a rule: its running
 // sum decays to rounding residue, which no bound can place against the cutoff.  The bare chain is
 // latency-bound (8 cycles per sample, 38 us for a block of 8192 with a window of 2048).
-// Replaying every block, which this replaces, took 172 us and the search through its stored values 118 us
-// on the same batch (288 us per call; now 104 us).
+// Replaying every block of every clip and searching the stored values, as an earlier version did, took 288 us per call
+// on this batch; now 52 us where no clip needs a replay, 104 to 171 us (over the signals) where most do.
+// Where every block is replayed (the rule in launch_nsr and region_kernel's `full`) the call costs, against that
+// version: the same batch with a window of 200 193 for 376 us, 512 clips of 10 s with a window of 16 267 for 497 us, 10
+// minutes in one clip with a window of 200 116 for 167 us and without resets 101 for 113 ms; the blocks replayed by
+// each clip's own CTA took 1322, 2047 and 30703 us and 174 ms.
 #include <cfloat>
 #include <climits>
 
@@ -37,14 +42,26 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kSub = 64;                       // samples per energy chunk
 constexpr int kUnit = kThreads / 32 * 1024;    // samples per CTA step of the energy pass
-constexpr int kChains = 8;                     // reset blocks replayed side by side, one per lane of warp 0
-constexpr int kTile = 256;                     // samples of each block per replay step
-constexpr int kPitch = kTile + 4;              // the 8 chain lanes' 16-byte reads fall in distinct banks
-constexpr size_t kReplayBytes = size_t(2) * 3 * kChains * kPitch * sizeof(float);
+// A replay: reset blocks side by side (a lane of warp 0 each), samples of each block per step, and the pitch of a row
+// of them, at which the lanes' 16-byte reads, up to 8 samples past the row, fall in distinct banks.
+template <int CHAINS, int TILE>
+struct ReplayShape
+{
+    static constexpr int kChains = CHAINS, kTile = TILE, kPitch = TILE + 12;
+    static constexpr int kStagers = kThreads / 32 - 1;                    // warps that stage
+    static constexpr int kRows = (CHAINS + kStagers - 1) / kStagers;     // blocks per staging warp
+    static constexpr size_t kBytes = size_t(2) * 3 * CHAINS * kPitch * sizeof(float);
+};
+using OneShape = ReplayShape<kThreads / 32 - 1, 256>;    // region_kernel: one block, seldom a few
+using ManyShape = ReplayShape<28, 128>;                  // exact_kernel: two CTAs per SM
 constexpr int kRun = 1024, kRuns = 512;        // largest_window: samples per run, runs whose maxima are kept
+constexpr int kSearch = 512;                   // chunks that largest_window searches at most (30 us)
+constexpr double kLongChain = 49152.0;         // operations of a reset block's chain from which region_kernel replays none
+constexpr int kTallyShift = 36;                // ExactList::tally: clips above, reset blocks (2^36: 256 GB of floats) below
+constexpr int kMaxClips = 1 << 27;             // per launch
 constexpr int kScan = 16;                      // chunks per thread and step of the scan of the energies
 constexpr int kHeld = kScan * kThreads;        // prefix energies kept in shared memory until the first replay
-static_assert(kReplayBytes >= (kHeld + 1) * sizeof(double), "the replay buffers hold the prefix energies first");
+static_assert(OneShape::kBytes >= (kHeld + 1) * sizeof(double), "the replay buffers hold the prefix energies first");
 constexpr double kUlp = 1.0 / 16777216.0;      // 2^-24: relative rounding error of a float operation
 
 __device__ __forceinline__ float sq(float v) { return __fmul_rn(v, v); }
@@ -54,9 +71,11 @@ __device__ __forceinline__ float sq(float v) { return __fmul_rn(v, v); }
 // warp that halves the number of values a lane carries at every step (8 FP64 shuffles for 16 chunks).
 __global__ void __launch_bounds__(kThreads) energy_kernel(const float* __restrict__ src, uint32_t stride,
                                                           const int* __restrict__ len, double* __restrict__ energies,
-                                                          long long pitch, int n, int unitsPerSample)
+                                                          long long pitch, int n, int unitsPerSample,
+                                                          unsigned long long* __restrict__ tally)
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (blockIdx.x == 0 && threadIdx.x < 2) *RPPB_WR(tally + threadIdx.x) = 0ull;
     const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
     const long long units = (long long)n * unitsPerSample;
     for (long long w = blockIdx.x; w < units; w += gridDim.x)
@@ -105,23 +124,33 @@ __global__ void __launch_bounds__(kThreads) energy_kernel(const float* __restric
     }
 }
 
+// The reset blocks that a CTA replays side by side, and what the replay finds.
+template <int kChains>
+struct ReplayShared
+{
+    const float* x[kChains];             // the block's sample
+    int pre[kChains], start[kChains], end[kChains];   // the fresh sum begins at pre, the block is [start, end)
+    float low[kChains], high[kChains];   // an MMS at or above them is at or above the cutoff interval's ends
+    // first and last index at or above the interval's low end, with the MMS there, and its high end (-1: none)
+    int firstLow[kChains], lastLow[kChains], firstHigh[kChains], lastHigh[kChains];
+    float firstValue[kChains], lastValue[kChains];
+    float peak[kChains];                 // the largest MMS, -infinity when every MMS is NaN
+    __device__ __forceinline__ void set(int j, const float* sample, int L, int W, int st, int R)
+    {
+        x[j] = sample;
+        pre[j] = max(st - W + 1, 0);
+        start[j] = st;
+        end[j] = int(min((long long)L, (long long)st + R));
+    }
+};
+
 // What the CTA of region_kernel shares.
-struct RegionShared
+struct RegionShared : ReplayShared<OneShape::kChains>
 {
     double warp[kThreads / 32], warp2[kThreads / 32];
     double sums[3 * kSub];               // running sums of squares within the chunks a window enters and leaves
     float run[kRuns];                    // largest window energy of each run
     int hit, sure;
-    int list[kChains];                   // blocks to replay
-    // per replayed block: first and last index at or above the cutoff interval's low end (with the MMS
-    // there in the low word; last: index + 1) and its high end
-    unsigned long long firstLow[kChains], lastLow[kChains];
-    int firstHigh[kChains], lastHigh[kChains];
-    unsigned peak[kChains];              // float_key of the largest MMS
-    __device__ __forceinline__ int low_index(int j, bool last) const
-    {
-        return last ? int(lastLow[j] >> 32) - 1 : int(firstLow[j] >> 32) & INT_MAX;
-    }
 };
 
 // One sample and its parameters.
@@ -135,6 +164,7 @@ struct Clip
     int chunks;
     double slack;         // absolute error of a difference of two entries of P
     double top;           // upper bound of every window energy
+    bool longChain;       // a replay costs more here than in exact_kernel
     __device__ __forceinline__ int pre(int st) const { return max(st - W + 1, 0); }
     __device__ __forceinline__ double prefix(int c) const { return *RPPB_RD(P + c); }
     // every window ending in chunk c lies inside these chunks
@@ -164,54 +194,48 @@ struct Clip
     }
 };
 
-// Replays the `m` reset blocks of sh.list exactly and fills sh's results for the cutoff interval
-// [low, high].  Lane j of warp 0 runs block j's chain from squares that the other seven warps stage in
-// shared memory one tile ahead; they also compare the MMS values one tile behind.  A square of zero
-// stands for "nothing enters / leaves": sum + 0 and sum - 0 == sum exactly.
-__device__ void replay(Clip& clip, RegionShared& sh, float* buf, int m, double low, double high)
+// Replays the first `m` reset blocks of sh exactly and fills sh's results.  Lane j of warp 0 runs block j's chain
+// from squares that the other warps, kRows blocks each, stage in shared memory one tile ahead; they also take the MMS
+// values one tile behind: the maximum, and (kEnds) the ends against the cutoff's interval.  A square of zero stands
+// for "nothing enters / leaves": sum + 0 and sum - 0 == sum exactly.
+template <class Shape, bool kEnds, int kChains>
+__device__ void replay(ReplayShared<kChains>& sh, float* buf, int m, int W, float meanFactor)
 {
+    constexpr int kTile = Shape::kTile, kRows = Shape::kRows, kLoads = kTile / 32, kAhead = 1024;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    auto row = [&](int slot, int what, int j) { return buf + ((slot * 3 + what) * kChains + j) * kPitch; };
-    auto start = [&](int j) { return sh.list[j] * clip.R; };
-    auto end = [&](int st) { return int(min((long long)clip.L, (long long)st + clip.R)); };
-    clip.P = clip.all;   // the buffers below take the place of the copy in shared memory
-    if (threadIdx.x < kChains)
+    auto row = [&](int slot, int what, int j) { return buf + ((slot * 3 + what) * Shape::kChains + j) * Shape::kPitch; };
+    if (threadIdx.x < m)
     {
-        sh.firstLow[threadIdx.x] = ~0ull;
-        sh.lastLow[threadIdx.x] = 0ull;
-        sh.firstHigh[threadIdx.x] = INT_MAX;
-        sh.lastHigh[threadIdx.x] = -1;
-        sh.peak[threadIdx.x] = float_key(-FLT_MAX);
-    }
-    if (threadIdx.x < m)   // the block's samples, ahead of the staging
-    {
-        const int st = start(threadIdx.x);
-        l2_prefetch(clip.x + clip.pre(st), clip.x + end(st));
+        const int j = threadIdx.x;   // the block's samples travel to L2 kAhead ahead of the staging
+        l2_prefetch(sh.x[j] + sh.pre[j], sh.x[j] + min((long long)sh.end[j], (long long)sh.pre[j] + kAhead));
     }
     __syncthreads();
     int preMax = 0, blkMax = 0;
     for (int j = 0; j < m; ++j)
     {
-        const int st = start(j);
-        preMax = max(preMax, st - clip.pre(st));
-        blkMax = max(blkMax, end(st) - st);
+        preMax = max(preMax, sh.start[j] - sh.pre[j]);
+        blkMax = max(blkMax, sh.end[j] - sh.start[j]);
     }
     const int preTiles = (preMax + kTile - 1) / kTile, tiles = preTiles + (blkMax + kTile - 1) / kTile;
-    float sum = 0.0f;
-    for (int it = 0; it < tiles + 2; ++it)
+    if (warp == 0)
     {
-        if (warp == 0)
+        float sum = 0.0f;
+        for (int it = 0; it < tiles + 2; ++it)
         {
             const int t = it - 1, slot = t & 1;
             if (t >= 0 && t < tiles && lane < m)
             {
-                const float* in = row(slot, 0, lane);
+                // two quads ahead of the chain
+                const float4* in = reinterpret_cast<const float4*>(row(slot, 0, lane));
+                float4 a0 = in[0], a1 = in[1];
                 if (t < preTiles)
                 {
 #pragma unroll 8
-                    for (int k = 0; k < kTile; k += 4)
+                    for (int k = 0; k < kTile / 4; ++k)
                     {
-                        const float4 a = *reinterpret_cast<const float4*>(in + k);
+                        const float4 a = a0;
+                        a0 = a1;
+                        a1 = in[k + 2];
                         sum = __fadd_rn(sum, a.x);
                         sum = __fadd_rn(sum, a.y);
                         sum = __fadd_rn(sum, a.z);
@@ -220,92 +244,178 @@ __device__ void replay(Clip& clip, RegionShared& sh, float* buf, int m, double l
                 }
                 else
                 {
-                    const float* out = row(slot, 1, lane);
-                    float* val = row(slot, 2, lane);
+                    const float4* out = reinterpret_cast<const float4*>(row(slot, 1, lane));
+                    float4* val = reinterpret_cast<float4*>(row(slot, 2, lane));
+                    float4 o0 = out[0], o1 = out[1];
 #pragma unroll 8
-                    for (int k = 0; k < kTile; k += 4)
+                    for (int k = 0; k < kTile / 4; ++k)
                     {
-                        const float4 a = *reinterpret_cast<const float4*>(in + k);
-                        const float4 o = *reinterpret_cast<const float4*>(out + k);
+                        const float4 a = a0, o = o0;
+                        a0 = a1;
+                        o0 = o1;
+                        a1 = in[k + 2];
+                        o1 = out[k + 2];
                         float4 v;
                         sum = __fadd_rn(sum, a.x);
-                        v.x = __fmul_rn(sum, clip.meanFactor);
+                        v.x = __fmul_rn(sum, meanFactor);
                         sum = __fsub_rn(sum, o.x);
                         sum = __fadd_rn(sum, a.y);
-                        v.y = __fmul_rn(sum, clip.meanFactor);
+                        v.y = __fmul_rn(sum, meanFactor);
                         sum = __fsub_rn(sum, o.y);
                         sum = __fadd_rn(sum, a.z);
-                        v.z = __fmul_rn(sum, clip.meanFactor);
+                        v.z = __fmul_rn(sum, meanFactor);
                         sum = __fsub_rn(sum, o.z);
                         sum = __fadd_rn(sum, a.w);
-                        v.w = __fmul_rn(sum, clip.meanFactor);
+                        v.w = __fmul_rn(sum, meanFactor);
                         sum = __fsub_rn(sum, o.w);
-                        *reinterpret_cast<float4*>(val + k) = v;
+                        val[k] = v;
                     }
                 }
+            }
+            __syncthreads();
+        }
+        __syncthreads();
+        return;
+    }
+    float a[kRows][kLoads], o[kRows][kLoads];   // samples entering and leaving, on their way
+    auto load = [&](int it) {
+        const bool fresh = it < preTiles;
+#pragma unroll
+        for (int r = 0; r < kRows; ++r)
+        {
+            const int j = warp - 1 + r * Shape::kStagers;
+            if (j >= m) break;
+            const int st = sh.start[j], from = fresh ? sh.pre[j] + it * kTile : st + (it - preTiles) * kTile;
+            // of the tile's samples the block has those below `left`, and those from `kept` on leave the window
+            const int left = (fresh ? st : sh.end[j]) - from;
+            const long long kept = (long long)W - 1 - from;
+            const float* x = sh.x[j] + from;
+            if (it % (kAhead / kTile) == 0 && lane == 0)
+            {
+                const long long ahead = (long long)from + kAhead;
+                l2_prefetch(sh.x[j] + ahead, sh.x[j] + min(ahead + kAhead, (long long)sh.end[j]));
+            }
+            if (left >= kTile && (fresh || kept <= 0))   // a whole tile: no comparison per sample
+            {
+#pragma unroll
+                for (int k = 0; k < kLoads; ++k) a[r][k] = __ldg(RPPB_RD(x + lane + 32 * k));
+                if (fresh) continue;
+                const float* gone = x + lane - W + 1;
+#pragma unroll
+                for (int k = 0; k < kLoads; ++k) o[r][k] = __ldg(RPPB_RD(gone + 32 * k));
+                continue;
+            }
+#pragma unroll
+            for (int k = 0; k < kLoads; ++k)
+            {
+                const int i = lane + 32 * k;
+                a[r][k] = i < left ? __ldg(RPPB_RD(x + i)) : 0.0f;
+                o[r][k] = !fresh && i < left && i >= kept ? __ldg(RPPB_RD(x + (i - W + 1))) : 0.0f;
             }
         }
-        else
+    };
+    // what each lane has seen of its values, in ascending order
+    float peak[kRows], firstValue[kRows], lastValue[kRows];
+    int firstLow[kRows], lastLow[kRows], firstHigh[kRows], lastHigh[kRows];
+#pragma unroll
+    for (int r = 0; r < kRows; ++r)
+    {
+        peak[r] = -INFINITY;
+        firstLow[r] = firstHigh[r] = INT_MAX;
+        lastLow[r] = lastHigh[r] = -1;
+        firstValue[r] = lastValue[r] = 0.f;
+    }
+    load(0);
+    for (int it = 0; it < tiles + 2; ++it)
+    {
+        if (it < tiles)
         {
-            const int first = threadIdx.x - 32, step = kThreads - 32, count = m * kTile;
-            if (it < tiles)
+#pragma unroll
+            for (int r = 0; r < kRows; ++r)
             {
-                const int slot = it & 1;
-#pragma unroll 2
-                for (int e = first; e < count; e += step)
-                {
-                    const int j = e / kTile, t = e % kTile, st = start(j);
-                    if (it < preTiles)
-                    {
-                        const int i = clip.pre(st) + it * kTile + t;
-                        row(slot, 0, j)[t] = i < st ? sq(__ldg(RPPB_RD(clip.x + i))) : 0.0f;
-                    }
-                    else
-                    {
-                        const long long i = (long long)st + (it - preTiles) * kTile + t;
-                        const long long o = i - clip.W + 1;
-                        const bool live = i < end(st);
-                        row(slot, 0, j)[t] = live ? sq(__ldg(RPPB_RD(clip.x + i))) : 0.0f;
-                        row(slot, 1, j)[t] = live && o >= 0 ? sq(__ldg(RPPB_RD(clip.x + o))) : 0.0f;
-                    }
-                }
+                const int j = warp - 1 + r * Shape::kStagers;
+                if (j >= m) break;
+                float* in = row(it & 1, 0, j) + lane;
+#pragma unroll
+                for (int k = 0; k < kLoads; ++k) in[32 * k] = sq(a[r][k]);
+                if (it < preTiles) continue;
+                float* out = row(it & 1, 1, j) + lane;
+#pragma unroll
+                for (int k = 0; k < kLoads; ++k) out[32 * k] = sq(o[r][k]);
             }
-            const int done = it - 2;
-            if (done >= preTiles)
+            if (it + 1 < tiles) load(it + 1);
+        }
+        const int done = it - 2;
+        if (done >= preTiles)
+        {
+#pragma unroll
+            for (int r = 0; r < kRows; ++r)
             {
-                // a warp's 32 consecutive values belong to one block (kTile and the step are multiples of 32)
-                for (int e = first; e < count; e += step)
+                const int j = warp - 1 + r * Shape::kStagers;
+                if (j >= m) break;
+                const float* val = row(done & 1, 2, j) + lane;
+                const int v0 = sh.start[j] + (done - preTiles) * kTile, left = sh.end[j] - v0;
+                if (!kEnds && left >= kTile)
                 {
-                    const int j = e / kTile, t = e % kTile;
-                    const long long i = (long long)start(j) + (done - preTiles) * kTile + t;
-                    const bool live = i < end(start(j));
-                    const float v = live ? row(done & 1, 2, j)[t] : -FLT_MAX;
-                    const unsigned atLow = __ballot_sync(0xffffffffu, live && double(v) >= low);
-                    const unsigned atHigh = __ballot_sync(0xffffffffu, live && double(v) >= high);
-                    const float mx = warp_max(fmaxf(-FLT_MAX, v));
-                    const unsigned long long bits = __float_as_uint(v);
-                    const unsigned long long at = (unsigned long long)(i);
-                    if (lane == __ffs(atLow) - 1) atomicMin(&sh.firstLow[j], at << 32 | bits);
-                    if (lane == 31 - __clz(atLow)) atomicMax(&sh.lastLow[j], (at + 1) << 32 | bits);
-                    if (lane == 0)
+#pragma unroll
+                    for (int k = 0; k < kLoads; ++k) peak[r] = fmaxf(peak[r], val[32 * k]);
+                    continue;
+                }
+                const float low = sh.low[j], high = sh.high[j];
+#pragma unroll
+                for (int k = 0; k < kLoads; ++k)
+                {
+                    const int i = lane + 32 * k;
+                    const float v = i < left ? val[32 * k] : NAN;   // a NaN takes part in nothing
+                    peak[r] = fmaxf(peak[r], v);
+                    if (kEnds && v >= low)
                     {
-                        atomicMax(&sh.peak[j], float_key(mx));
-                        if (atHigh)
+                        lastLow[r] = v0 + i;
+                        lastValue[r] = v;
+                        if (firstLow[r] == INT_MAX)
                         {
-                            atomicMin(&sh.firstHigh[j], int(i) + __ffs(atHigh) - 1);
-                            atomicMax(&sh.lastHigh[j], int(i) + 31 - __clz(atHigh));
+                            firstLow[r] = v0 + i;
+                            firstValue[r] = v;
                         }
+                    }
+                    if (kEnds && v >= high)
+                    {
+                        lastHigh[r] = v0 + i;
+                        firstHigh[r] = min(firstHigh[r], v0 + i);
                     }
                 }
             }
         }
         __syncthreads();
     }
+#pragma unroll
+    for (int r = 0; r < kRows; ++r)
+    {
+        const int j = warp - 1 + r * Shape::kStagers;
+        if (j >= m) break;
+        const float top = warp_max(peak[r]);
+        if (lane == 0) sh.peak[j] = top;
+        if constexpr (kEnds)
+        {
+            const int f = __reduce_min_sync(0xffffffffu, firstLow[r]), l = __reduce_max_sync(0xffffffffu, lastLow[r]);
+            const int fh = __reduce_min_sync(0xffffffffu, firstHigh[r]), lh = __reduce_max_sync(0xffffffffu, lastHigh[r]);
+            if (f == firstLow[r]) sh.firstValue[j] = firstValue[r];   // one lane, unless there is none
+            if (l == lastLow[r]) sh.lastValue[j] = lastValue[r];
+            if (lane == 0)
+            {
+                sh.firstLow[j] = f == INT_MAX ? -1 : f;
+                sh.lastLow[j] = l;
+                sh.firstHigh[j] = fh == INT_MAX ? -1 : fh;
+                sh.lastHigh[j] = lh;
+            }
+        }
+    }
+    __syncthreads();
 }
 
 constexpr int kNone = -1;        // no MMS reaches the cutoff
 constexpr int kUnsettled = -2;   // an exact MMS lies inside the cutoff's interval
-constexpr int kGiveUp = -3;      // too many candidates: replay everything
+constexpr int kGiveUp = -3;      // too many candidates: exact_kernel replays every block
 
 // An exact MMS inside the cutoff's interval: the first (last) one at or above its low end.
 struct Open
@@ -402,17 +512,22 @@ __device__ int find_end(Clip& clip, RegionShared& sh, float* buf, double low, do
         }
         if (sh.sure) return at;
         // undecided: the exact values of that sample's block
-        if (++replays > 2) return kGiveUp;
+        if (clip.longChain || ++replays > 2) return kGiveUp;
         const int k = at / clip.R;
-        if (tid == 0) sh.list[0] = k;
+        if (tid == 0)
+        {
+            sh.set(0, clip.x, clip.L, clip.W, k * clip.R, clip.R);
+            sh.low[0] = __double2float_ru(low);
+            sh.high[0] = __double2float_ru(high);
+        }
+        clip.P = clip.all;   // the replay's buffers take the place of the copy in shared memory
         __syncthreads();
-        replay(clip, sh, buf, 1, low, high);
-        const bool any = sh.lastLow[0] != 0ull;
-        const int lo = sh.low_index(0, kLast), hi = kLast ? sh.lastHigh[0] : sh.firstHigh[0];
+        replay<OneShape, true>(sh, buf, 1, clip.W, clip.meanFactor);
+        const int lo = kLast ? sh.lastLow[0] : sh.firstLow[0], hi = kLast ? sh.lastHigh[0] : sh.firstHigh[0];
         open.index = lo;
-        open.value = __uint_as_float(unsigned(kLast ? sh.lastLow[0] : sh.firstLow[0]));
+        open.value = kLast ? sh.lastValue[0] : sh.firstValue[0];
         __syncthreads();
-        if (any) return lo == hi ? lo : kUnsettled;
+        if (lo >= 0) return lo == hi ? lo : kUnsettled;
         const long long next = kLast ? (long long)k * clip.R - 1 : (long long)(k + 1) * clip.R;
         if (next < 0 || next >= clip.L) return kNone;
         edge = int(next);
@@ -424,13 +539,22 @@ __device__ int find_end(Clip& clip, RegionShared& sh, float* buf, double low, do
 // cutoff's interval: the chunks bound it to 3 % (64 samples of 2048).  Each warp takes 128 samples at a
 // time, wherever the chunks allow a window of at least `least`: the window energy before them plus the
 // running sum of the squares entering less those leaving (in float; the steps are independent).
-// sh.run[r] = the largest of run r (kRuns runs at most).
+// sh.run[r] = the largest of run r (kRuns runs at most).  Negative: too many chunks to search (a clip of steady level).
 __device__ double largest_window(const Clip& clip, RegionShared& sh, double least)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     auto square = [&](long long i) { return i >= 0 && i < clip.L ? sq(__ldg(RPPB_RD(clip.x + i))) : 0.0f; };
     for (int r = threadIdx.x; r < kRuns; r += kThreads) sh.run[r] = 0.0f;
+    if (threadIdx.x == 0) sh.hit = 0;
     __syncthreads();
+    int chunks = 0;
+    for (int c = threadIdx.x; c < clip.chunks; c += kThreads) chunks += clip.upper(c) >= least;
+    chunks = __reduce_add_sync(0xffffffffu, chunks);
+    if (lane == 0 && chunks > 0) atomicAdd(&sh.hit, chunks);
+    __syncthreads();
+    const bool many = sh.hit > kSearch;
+    __syncthreads();
+    if (many) return -1.0;
     float best = 0.0f;
     for (int c = 2 * warp; c < clip.chunks; c += 2 * (kThreads / 32))
     {
@@ -480,78 +604,71 @@ __device__ double largest_window(const Clip& clip, RegionShared& sh, double leas
     return all;
 }
 
-// The largest MMS, by replaying the blocks that `may(k)` (uniform over the CTA) admits.
-template <class May>
-__device__ float exact_peak(Clip& clip, RegionShared& sh, float* buf, int blocks, May may)
+// What the clips whose ends region_kernel does not settle leave for exact_kernel.
+struct ExactList
 {
-    float peak = -FLT_MAX;
-    int m = 0;
-    for (int k = 0; k <= blocks; ++k)
+    unsigned long long* tally;   // entries << kTallyShift | their reset blocks, then the blocks claimed; zeroed by energy_kernel
+    int* clip;                   // entry -> clip
+    long long* first;            // entry -> its first block in blockMax
+    int* done;                   // entry -> blocks replayed
+    float* blockMax;             // largest MMS of each block, NaN when all are
+};
+
+__device__ __forceinline__ void write_region(int first, int last, int W, int b, int* outBegin, int* outLength)
+{
+    int detectBegin = 0, detectLength = 0;
+    if (first >= 0)
     {
-        if (k < blocks && may(k))
+        detectBegin = first;
+        detectLength = last - first + 1;
+        if (detectBegin != 0 && detectLength != 0)
         {
-            if (threadIdx.x == 0) sh.list[m] = k;
-            ++m;
-        }
-        if (m == kChains || (k == blocks && m > 0))
-        {
-            __syncthreads();
-            replay(clip, sh, buf, m, double(INFINITY), double(INFINITY));
-            for (int j = 0; j < m; ++j) peak = fmaxf(peak, key_float(sh.peak[j]));
-            __syncthreads();
-            m = 0;
+            const int newBegin = max(detectBegin - (W - 1), 0);
+            detectLength += detectBegin - newBegin;
+            detectBegin = newBegin;
         }
     }
-    return peak;
-}
-
-// Both ends by replaying blocks from either side until one reaches the exact cutoff.
-__device__ void replay_ends(Clip& clip, RegionShared& sh, float* buf, int blocks, double cut, int& first, int& last)
-{
-    first = last = -1;
-    for (int dir = 0; dir < 2; ++dir)
-        for (int g = 0; g < blocks; g += kChains)
-        {
-            const int m = min(kChains, blocks - g);
-            if (threadIdx.x < m) sh.list[threadIdx.x] = dir ? blocks - 1 - g - int(threadIdx.x) : g + int(threadIdx.x);
-            __syncthreads();
-            replay(clip, sh, buf, m, cut, cut);
-            int at = -1;
-            for (int j = 0; j < m && at < 0; ++j)
-                if (sh.lastLow[j] != 0ull) at = sh.low_index(j, dir != 0);
-            __syncthreads();
-            if (at < 0) continue;
-            (dir ? last : first) = at;
-            break;
-        }
+    *RPPB_WR(outBegin + b) = detectBegin;
+    *RPPB_WR(outLength + b) = detectLength;
 }
 
 __global__ void __launch_bounds__(kThreads) region_kernel(const float* __restrict__ src, uint32_t stride,
                                                           const int* __restrict__ len, int windowLength, int reset,
                                                           float referencePower, float cutOff, double* __restrict__ energies,
-                                                          long long pitch, int* __restrict__ outBegin,
-                                                          int* __restrict__ outLength)
+                                                          long long pitch, bool intervals, ExactList exact,
+                                                          int* __restrict__ outBegin, int* __restrict__ outLength)
 {
-    // kReplayBytes: the prefix energies, then squares entering, squares leaving and MMS in two slots
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // OneShape::kBytes: the prefix energies, then squares entering, squares leaving and MMS in two slots
     extern __shared__ __align__(16) float buf[];
     __shared__ RegionShared sh;
     const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int L = min(*RPPB_RD(len + b), int(stride));
-    grid_dependency_wait();   // the chunk energies
+    grid_dependency_wait();   // the chunk energies, the zeroed tally
     if (L <= 0)
     {
-        if (tid == 0)
-        {
-            *RPPB_WR(outBegin + b) = 0;
-            *RPPB_WR(outLength + b) = 0;
-        }
+        if (tid == 0) write_region(-1, -1, windowLength, b, outBegin, outLength);
         return;
     }
+    // leaves the clip to exact_kernel
+    auto pass_on = [&](int blocks) {
+        const unsigned long long t =
+            atomicAdd(RPPB_WR(dependency_result(exact.tally)), 1ull << kTallyShift | (unsigned long long)blocks);
+        const int e = int(t >> kTallyShift);
+        *RPPB_WR(exact.clip + e) = b;
+        *RPPB_WR(exact.first + e) = (long long)(t & ((1ull << kTallyShift) - 1));
+        *RPPB_WR(exact.done + e) = 0;
+    };
     double* P = dependency_result(energies) + b * pitch;
     double* held = reinterpret_cast<double*>(buf);
     Clip clip{src + size_t(b) * stride, L, windowLength, reset == -1 ? L : reset,
-              __fdiv_rn(1.0f, float(windowLength)), P, P, (L + kSub - 1) / kSub, 0.0, 0.0};
+              __fdiv_rn(1.0f, float(windowLength)), P, P, (L + kSub - 1) / kSub, 0.0, 0.0, false};
     const int blocks = int(((long long)L + clip.R - 1) / clip.R);
+    if (!intervals)
+    {
+        if (tid == 0) pass_on(blocks);
+        return;
+    }
 
     // energies -> prefix energies, in place: a warp takes kScan rows of 32 chunks, which it scans side by side
     double total = 0.0;
@@ -606,9 +723,10 @@ __global__ void __launch_bounds__(kThreads) region_kernel(const float* __restric
     int first = -1, last = -1;
     const bool peakRef = referencePower == 0.0f;
     const double ops = double(windowLength) + 2.0 * double(min(clip.R, L));
-    // Intervals help where the chunks resolve the window, the chain's rounding bound is small and every
-    // number is a normal one; elsewhere (and when they do not settle the ends) every block is replayed.
-    bool full = !(total <= 1e37) || windowLength < 4 * kSub || clip.R < kSub || ops * kUlp > 1.0 / 16;
+    clip.longChain = ops > kLongChain;
+    // Intervals help where the chain's rounding bound is small and every number is a normal one; elsewhere (and
+    // when they do not settle the ends) every block is replayed.
+    bool full = !(total <= 1e37) || clip.R < kSub || ops * kUlp > 1.0 / 16;
     if (total == 0.0)
     {
         // every square is zero and so is every MMS
@@ -661,30 +779,57 @@ __global__ void __launch_bounds__(kThreads) region_kernel(const float* __restric
         else
         {
             // 0: the interval the chunks give, 1: a tighter one, 2: the exact cutoff
-            for (int stage = 0;; ++stage)
+            for (int stage = 0;;)
             {
                 Open open{};
                 if (first < 0) first = find_end<false>(clip, sh, buf, low, high, open);
                 last = first < 0 ? first : find_end<true>(clip, sh, buf, low, high, open);
                 if (last != kUnsettled || !peakRef || stage == 2) break;
-                if (stage == 0)
+                bool found = true;
+                do   // until the open value is outside the interval
                 {
-                    const double tol = 1e-5 * clip.top;
-                    const double peak = largest_window(clip, sh, lo - clip.slack - 2.0 * (err + tol));
-                    peakLow = peak - tol - err;
-                    cutoff_interval(peak + tol + err);
-                }
-                else
+                    if (stage == 0)
+                    {
+                        const double tol = 1e-5 * clip.top;
+                        const double peak = largest_window(clip, sh, lo - clip.slack - 2.0 * (err + tol));
+                        found = peak >= 0.0;
+                        if (!found) break;
+                        peakLow = peak - tol - err;
+                        cutoff_interval(peak + tol + err);
+                    }
+                    else
+                    {
+                        // from the blocks whose energies allow the maximum, unless they are too many
+                        if (tid == 0) sh.hit = 0;
+                        __syncthreads();
+                        for (int k = tid; k < blocks; k += kThreads)
+                        {
+                            const int st = k * clip.R, en = int(min((long long)L, (long long)st + clip.R));
+                            bool any = false;
+                            for (int r = st / kRun; !any && r <= (en - 1) / kRun; ++r)
+                                any = r >= kRuns || sh.run[r] + 1e-5 * clip.top + err >= peakLow;
+                            if (!any) continue;
+                            const int at = atomicAdd(&sh.hit, 1);
+                            if (at < OneShape::kChains) sh.set(at, clip.x, L, clip.W, st, clip.R);
+                        }
+                        __syncthreads();
+                        const int m = sh.hit;
+                        found = m <= OneShape::kChains;
+                        if (!found) break;
+                        clip.P = clip.all;
+                        replay<OneShape, false>(sh, buf, m, clip.W, clip.meanFactor);
+                        float peak = -FLT_MAX;
+                        for (int j = 0; j < m; ++j)
+                            peak = fmaxf(peak, sh.peak[j]);
+                        __syncthreads();
+                        low = high = double(__fmul_rn(peak, cutOff));
+                    }
+                    ++stage;
+                } while (stage < 2 && double(open.value) >= low && double(open.value) < high);
+                if (!found)
                 {
-                    // from the blocks whose energies allow the maximum
-                    const float peak = exact_peak(clip, sh, buf, blocks, [&](int k) {
-                        const int st = k * clip.R, en = int(min((long long)L, (long long)st + clip.R));
-                        bool any = false;
-                        for (int r = st / kRun + tid; r <= (en - 1) / kRun; r += kThreads)
-                            any = any || r >= kRuns || sh.run[r] + 1e-5 * clip.top + err >= peakLow;
-                        return __syncthreads_or(any) != 0;
-                    });
-                    low = high = double(__fmul_rn(peak, cutOff));
+                    first = kGiveUp;
+                    break;
                 }
                 if (double(open.value) < high) continue;
                 // the open value is the end: everything before (after) it is below the interval's old low end
@@ -698,40 +843,158 @@ __global__ void __launch_bounds__(kThreads) region_kernel(const float* __restric
             full = first < kNone || last < kNone;
         }
     }
-    if (full)
+    if (tid != 0) return;
+    if (full) pass_on(blocks);
+    else write_region(first, last, windowLength, b, outBegin, outLength);
+}
+
+// The clips of the list: their reset blocks, dealt to the CTAs of the whole grid a few at a time, are replayed for
+// their maxima; the CTA that replays a clip's last block then has the cutoff, and replays the first and the last block
+// that reach it for the ends.  No CTA waits for another.  Bound by the chains' latency (10 cycles per sample) until
+// 8288 blocks are in flight, then by the issue of the staging.  28 blocks of 128 samples per CTA: 14 of 256 took 1746
+// instead of 1470 us on 512000 blocks of 32 samples, as much elsewhere; 28 of 64 took 359 instead of 267 us on 8200
+// blocks of 8192.
+__global__ void __launch_bounds__(kThreads, 2) exact_kernel(const float* __restrict__ src, uint32_t stride,
+                                                            const int* __restrict__ len, int windowLength, int reset,
+                                                            float referencePower, float cutOff, ExactList list,
+                                                            int* __restrict__ outBegin, int* __restrict__ outLength)
+{
+    constexpr int kChains = ManyShape::kChains;
+    static_assert(kChains <= 32, "a lane each");
+    static_assert(OneShape::kBytes <= ManyShape::kBytes && OneShape::kChains <= kChains, "the ends' replay");
+    extern __shared__ __align__(16) float buf[];   // ManyShape::kBytes
+    __shared__ ReplayShared<kChains> sh;
+    __shared__ int s_entry[kChains], s_last[kChains];   // per replayed block: its entry; the entry again when it was its last
+    __shared__ int s_clip[kChains], s_first, s_final;
+    __shared__ float s_max[kThreads / 32];
+    __shared__ long long s_next;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const float meanFactor = __fdiv_rn(1.0f, float(windowLength));
+    grid_dependency_wait();
+    const unsigned long long tally = *RPPB_RD(dependency_result(list.tally));
+    const long long total = (long long)(tally & ((1ull << kTallyShift) - 1));
+    if (total == 0) return;
+    const int entries = int(tally >> kTallyShift);
+    const int* clips = dependency_result(list.clip);
+    const long long* firsts = dependency_result(list.first);
+    const int per = int(min((long long)kChains, (total + gridDim.x - 1) / gridDim.x));   // blocks per CTA step
+    auto samples = [&](int b) { return min(*RPPB_RD(len + b), int(stride)); };
+    auto block_len = [&](int L) { return reset == -1 ? L : reset; };
+    auto block_count = [&](int L) { return int(((long long)L + block_len(L) - 1) / block_len(L)); };
+    for (;;)
     {
-        float base = referencePower;
-        if (peakRef) base = exact_peak(clip, sh, buf, blocks, [](int) { return true; });
-        replay_ends(clip, sh, buf, blocks, double(__fmul_rn(base, cutOff)), first, last);
-    }
-    if (tid == 0)
-    {
-        int detectBegin = 0, detectLength = 0;
-        if (first >= 0)
+        // claimed, not dealt: a CTA that has finished a clip would stay behind, and so finish the next ones too
+        if (tid == 0) s_next = (long long)atomicAdd(RPPB_WR(dependency_result(list.tally) + 1), (unsigned long long)per);
+        __syncthreads();
+        const long long w = s_next;
+        if (w >= total) break;
+        const int m = int(min((long long)per, total - w));
+        if (tid < m)
         {
-            detectBegin = first;
-            detectLength = last - first + 1;
-            if (detectBegin != 0 && detectLength != 0)
-            {
-                const int newBegin = max(detectBegin - (windowLength - 1), 0);
-                detectLength += detectBegin - newBegin;
-                detectBegin = newBegin;
-            }
+            const int e = ragged_find(firsts, entries, w + tid), b = *RPPB_RD(clips + e);
+            const int L = samples(b), R = block_len(L);
+            s_entry[tid] = e;
+            sh.set(tid, src + size_t(b) * stride, L, windowLength, int(w + tid - *RPPB_RD(firsts + e)) * R, R);
         }
-        *RPPB_WR(outBegin + b) = detectBegin;
-        *RPPB_WR(outLength + b) = detectLength;
+        __syncthreads();
+        replay<ManyShape, false>(sh, buf, m, windowLength, meanFactor);
+        if (tid < m)
+        {
+            const int e = s_entry[tid];
+            *RPPB_WR(list.blockMax + (w + tid)) = sh.peak[tid] == -INFINITY ? NAN : sh.peak[tid];
+            __threadfence();   // the maximum before the count
+            const int before = atomicAdd(RPPB_WR(list.done + e), 1);
+            s_last[tid] = before + 1 == block_count(samples(*RPPB_RD(clips + e))) ? e : -1;
+        }
+        __syncthreads();
+        // the clips whose last block this was, as many at a time as their end blocks fit side by side
+        int ends = 0;    // end blocks gathered
+        auto finish = [&] {
+            __syncthreads();
+            replay<OneShape, true>(sh, buf, ends, windowLength, meanFactor);
+            // a clip's blocks are neighbours, its first one carries the clip
+            if (tid < ends && s_clip[tid] >= 0)
+            {
+                const int other = tid + 1 < ends && s_clip[tid + 1] < 0 ? tid + 1 : tid;
+                write_region(sh.firstLow[tid], sh.lastLow[other], windowLength, s_clip[tid], outBegin, outLength);
+            }
+            __syncthreads();
+            ends = 0;
+        };
+        for (int j = 0; j < m; ++j)
+        {
+            const int e = s_last[j];
+            if (e < 0) continue;
+            const int b = *RPPB_RD(clips + e), L = samples(b), R = block_len(L), blocks = block_count(L);
+            const float* maxima = list.blockMax + *RPPB_RD(firsts + e);
+            __threadfence();
+            float base = referencePower;
+            if (referencePower == 0.0f)
+            {
+                float peak = -FLT_MAX;
+                for (int k = tid; k < blocks; k += kThreads) peak = fmaxf(peak, __ldcg(RPPB_RD(maxima + k)));
+                peak = warp_max(peak);
+                if (lane == 0) s_max[warp] = peak;
+                __syncthreads();
+                base = s_max[0];
+                for (int i = 1; i < kThreads / 32; ++i) base = fmaxf(base, s_max[i]);
+            }
+            const float cut = __fmul_rn(base, cutOff);
+            if (tid == 0)
+            {
+                s_first = INT_MAX;
+                s_final = -1;
+            }
+            __syncthreads();
+            for (int k = tid; k < blocks; k += kThreads)
+                if (__ldcg(RPPB_RD(maxima + k)) >= cut)
+                {
+                    atomicMin(&s_first, k);
+                    atomicMax(&s_final, k);
+                }
+            __syncthreads();
+            const int first = s_first, final = s_final;
+            __syncthreads();   // s_first, s_final and s_max are free
+            if (final < 0)
+            {
+                if (tid == 0) write_region(-1, -1, windowLength, b, outBegin, outLength);
+                continue;
+            }
+            const int need = first == final ? 1 : 2;
+            if (ends + need > OneShape::kChains) finish();
+            if (tid < need)
+            {
+                const int at = ends + tid;
+                s_clip[at] = tid == 0 ? b : -1;
+                sh.set(at, src + size_t(b) * stride, L, windowLength, (tid == 0 ? first : final) * R, R);
+                sh.low[at] = sh.high[at] = cut;
+            }
+            ends += need;
+        }
+        if (ends > 0) finish();
     }
 }
 
 // prefix energies per sample: one more entry than chunks
 long long energy_pitch(uint32_t srcStride) { return (long long)(srcStride / kSub) + 2; }
 
+// reset blocks of the batch, at most
+size_t block_count(int n, uint32_t srcStride, int resetInterval)
+{
+    return resetInterval == -1 ? size_t(n) : size_t(n) * ((size_t(srcStride) + resetInterval - 1) / resetInterval);
+}
+
 }  // namespace
 
-size_t nsr_scratch_bytes(int n, uint32_t srcStride)
+size_t nsr_scratch_bytes(int n, uint32_t srcStride, int resetInterval)
 {
     Carver cv(nullptr);
+    cv.take<unsigned long long>(2);
     cv.take<double>(size_t(n) * energy_pitch(srcStride));
+    cv.take<int>(n);
+    cv.take<long long>(n);
+    cv.take<int>(n);
+    cv.take<float>(block_count(n, srcStride, resetInterval));
     return cv.used();
 }
 
@@ -740,19 +1003,38 @@ void launch_nsr(Handle& h, void* scratch, const NsrArgs& a)
     if (a.n <= 0) return;
     Carver cv(scratch);
     const long long pitch = energy_pitch(a.srcStride);
+    ExactList list;
+    list.tally = cv.take<unsigned long long>(2);
     double* energies = cv.take<double>(size_t(a.n) * pitch);
+    list.clip = cv.take<int>(a.n);
+    list.first = cv.take<long long>(a.n);
+    list.done = cv.take<int>(a.n);
+    list.blockMax = cv.take<float>(block_count(a.n, a.srcStride, a.resetInterval));
+    // the intervals' chunks have to resolve the window and the reset blocks; else exact_kernel takes every clip
+    const bool intervals = a.windowLength >= 4 * kSub && (a.resetInterval == -1 || a.resetInterval >= kSub);
     const int ups = int(a.srcStride / kUnit) + 1;
-    const long long units = (long long)a.n * ups;
-    const int grid = int(std::min<long long>(
-        units, persistent_grid(h, reinterpret_cast<const void*>(energy_kernel), kThreads, 0)));
-    energy_kernel<<<grid, kThreads, 0, h.stream()>>>(a.src, a.srcStride, a.len, energies, pitch, a.n, ups);
-    count_launch();
-    check_cuda(cudaGetLastError(), "energy_kernel");
-    persistent_grid(h, reinterpret_cast<const void*>(region_kernel), kThreads, kReplayBytes);   // shared-memory opt-in
-    launch_dependent(region_kernel, dim3(a.n), dim3(kThreads), kReplayBytes, h.stream(), "region_kernel", a.src,
-                     a.srcStride, a.len, a.windowLength, a.resetInterval, a.referencePower, a.cutOff, energies, pitch,
-                     a.begin, a.length);
-    count_launch();
+    for (int b0 = 0; b0 < a.n; b0 += kMaxClips)
+    {
+        const int n = std::min(a.n - b0, kMaxClips);
+        const float* src = a.src + size_t(b0) * a.srcStride;
+        const long long units = intervals ? (long long)n * ups : 1;
+        const int grid = int(std::min<long long>(
+            units, persistent_grid(h, reinterpret_cast<const void*>(energy_kernel), kThreads, 0)));
+        energy_kernel<<<grid, kThreads, 0, h.stream()>>>(src, a.srcStride, a.len + b0, energies, pitch,
+                                                         intervals ? n : 0, ups, list.tally);
+        count_launch();
+        check_cuda(cudaGetLastError(), "energy_kernel");
+        persistent_grid(h, reinterpret_cast<const void*>(region_kernel), kThreads, OneShape::kBytes);   // shared-memory opt-in
+        launch_dependent(region_kernel, dim3(n), dim3(kThreads), OneShape::kBytes, h.stream(), "region_kernel", src,
+                         a.srcStride, a.len + b0, a.windowLength, a.resetInterval, a.referencePower, a.cutOff, energies,
+                         pitch, intervals, list, a.begin + b0, a.length + b0);
+        count_launch();
+        const int exactGrid = persistent_grid(h, reinterpret_cast<const void*>(exact_kernel), kThreads, ManyShape::kBytes);
+        launch_dependent(exact_kernel, dim3(exactGrid), dim3(kThreads), ManyShape::kBytes, h.stream(), "exact_kernel", src,
+                         a.srcStride, a.len + b0, a.windowLength, a.resetInterval, a.referencePower, a.cutOff, list,
+                         a.begin + b0, a.length + b0);
+        count_launch();
+    }
 }
 
 }  // namespace rppb

@@ -101,8 +101,8 @@ struct NsrArgs
     float referencePower;
     int resetInterval;
 };
-// Prefix energies of the samples' 64-sample chunks (FP64).
-size_t nsr_scratch_bytes(int n, uint32_t srcStride);
+// Prefix energies of the samples' 64-sample chunks (FP64), the list of undecided samples and their reset blocks' maxima.
+size_t nsr_scratch_bytes(int n, uint32_t srcStride, int resetInterval);
 void launch_nsr(Handle& h, void* scratch, const NsrArgs& a);
 
 // Mel filter placement parameters (maxFreq already resolved: 0 -> sampleRate / 2).

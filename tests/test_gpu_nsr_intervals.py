@@ -1,5 +1,6 @@
 """non_silent_region_detection decides from energy intervals and replays a reset block's float chain only where
-they do not settle an end: inputs at the edges of that rule, whole numbers equal to the oracle's."""
+they do not settle an end, and every block where intervals do not help: inputs at the edges of that rule, whole numbers
+equal to the oracle's, and the replay of every block spread over the GPU."""
 import numpy as np
 import pytest
 
@@ -58,3 +59,70 @@ def test_region_equals_oracle(gpu, oracle, reset, window, ref, cut, pad):
                                              window, ref, reset, gpu) == 0
     np.testing.assert_array_equal(host(begin), b_ref)
     np.testing.assert_array_equal(host(length), l_ref)
+
+
+def detect(gpu, x, lens, window, reset, cut=-60.0, ref=0.0):
+    """(begin, length) on the host, and a repeatable call."""
+    begin = torch.full((len(lens),), -7, dtype=torch.int32, device="cuda")
+    length = torch.full((len(lens),), -7, dtype=torch.int32, device="cuda")
+    xd, ld, sd = dev(x), dev(lens), audio_desc(len(lens), x.shape[1])
+
+    def call():
+        assert audio.non_silent_region_detection(xd, sd, ld, begin, length, cut, window, ref, reset, gpu) == 0
+    call()
+    return host(begin), host(length), call
+
+
+# 262144 samples: the prefix energies that a CTA holds in shared memory; 524288: the runs whose maxima it keeps
+@pytest.mark.parametrize("reset,window,cut", [(8192, 2048, -60.0), (8192, 2048, 0.0), (8192, 2048, -0.02),
+                                              (8192, 200, -60.0), (-1, 2048, -60.0), (50000, 2048, -60.0)])
+def test_long_clips_equal_oracle(gpu, oracle, reset, window, cut):
+    r = np.random.default_rng(11)
+    lens = np.array([262143, 262144, 262145, 600000, 600001, 300], np.int32)
+    x = np.zeros((len(lens), 600001), np.float32)
+    for i, n in enumerate(lens):
+        x[i, n // 9:n - n // 7] = r.normal(0, 0.1, n - n // 7 - n // 9)   # silence at both ends
+    x[3, 540000:543000] *= 3.0                                           # the maximum past the kept runs
+    x[4, 1000:] = 0.1 * np.sin(np.arange(599001) * 0.05)                 # a steady level: every block may hold it
+    b_ref, l_ref = oracle.nsr(x, lens, cut, window, 0.0, reset)
+    begin, length, _ = detect(gpu, x, lens, window, reset, cut)
+    np.testing.assert_array_equal(begin, b_ref)
+    np.testing.assert_array_equal(length, l_ref)
+
+
+@pytest.mark.parametrize("reset,window,ref", [(8192, 100, 0.0), (8192, 3, 0.05), (32, 500, 0.0), (1, 2, 0.0)])
+def test_many_clips_with_every_block_replayed(gpu, oracle, reset, window, ref):
+    """More clips, and more blocks in a clip, than a CTA replays side by side; a clip with a NaN."""
+    r = np.random.default_rng(12)
+    n = 700
+    lens = r.integers(1, 9000 if reset == 1 else 40000, n).astype(np.int32)
+    x = np.zeros((n, int(lens.max())), np.float32)
+    for i, k in enumerate(lens):
+        x[i, k // 8:k - k // 6] = r.normal(0, 0.2, k - k // 6 - k // 8)
+    x[6, lens[6] // 2] = np.nan
+    with np.errstate(invalid="ignore"):
+        b_ref, l_ref = oracle.nsr(x, lens, -60.0, window, ref, reset)
+    begin, length, _ = detect(gpu, x, lens, window, reset, -60.0, ref)
+    np.testing.assert_array_equal(begin, b_ref)
+    np.testing.assert_array_equal(length, l_ref)
+
+
+def test_replay_of_every_block_is_spread_over_the_gpu(gpu):
+    """A long clip with a window just below the intervals' range: its 586 blocks replayed one after the other, a few
+    at a time, take some hundred times the call with a window just inside."""
+    x = np.random.default_rng(13).normal(0, 0.1, (1, 4800000)).astype(np.float32)
+    lens = np.array([4800000], np.int32)
+
+    def best(window):
+        call = detect(gpu, x, lens, window, 8192)[2]
+        times = []
+        for _ in range(7):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            call()
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times)
+
+    assert best(255) < 8 * best(256)
