@@ -96,6 +96,27 @@ __device__ __forceinline__ const long long* cache_prefix(const long long* prefix
     return s_cache;
 }
 
+// Exclusive scan of one value per thread of a CTA of whole warps: warp scans of the values and of the warps' totals
+// (each warp its own copy), one barrier.  s_total is shared; before it is used again all threads must have returned.
+__device__ __forceinline__ long long block_exclusive_scan(long long value, long long (&s_total)[32])
+{
+    const int t = threadIdx.x, lane = t & 31;
+    auto scan = [&](long long v) {
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
+        {
+            const long long u = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += u;
+        }
+        return v;
+    };
+    const long long incl = scan(value);
+    if (lane == 31) s_total[t >> 5] = incl;
+    __syncthreads();
+    const long long before = scan(lane < (t >> 5) ? s_total[lane] : 0);
+    return __shfl_sync(0xffffffffu, before, 31) + incl - value;
+}
+
 // One CTA of up to 1024 threads, a clip each (or several): prefix[0..n] = exclusive scan of count(b), and
 // zero[0..zeroWords) = 0 (the work counters of the kernel that follows).  It lets a kernel launched after it with
 // programmatic stream serialization (launch_dependent) start at once; that kernel runs its
@@ -107,29 +128,15 @@ __global__ void __launch_bounds__(1024) ragged_prefix_kernel(Count count, int n,
                                                              unsigned* __restrict__ zero, int zeroWords)
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const int t = threadIdx.x, lane = t & 31, threads = blockDim.x;
+    const int t = threadIdx.x, threads = blockDim.x;
     const int per = (n + threads - 1) / threads;
     const int b0 = min(n, t * per), b1 = min(n, b0 + per);
     const long long first = b0 < b1 ? count(b0) : 0;
     for (int i = t; i < zeroWords; i += threads) *RPPB_WR(zero + i) = 0u;
     long long sum = first;
     for (int b = b0 + 1; b < b1; ++b) sum += count(b);
-    // inclusive scans of the warp and of the warps' totals (each warp its own copy): one barrier
-    auto scan = [&](long long v) {
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1)
-        {
-            const long long u = __shfl_up_sync(0xffffffffu, v, o);
-            if (lane >= o) v += u;
-        }
-        return v;
-    };
     __shared__ long long s_total[32];
-    const long long incl = scan(sum);
-    if (lane == 31) s_total[t >> 5] = incl;
-    __syncthreads();
-    const long long before = scan(lane < (t >> 5) ? s_total[lane] : 0);
-    long long run = __shfl_sync(0xffffffffu, before, 31) + incl - sum;
+    long long run = block_exclusive_scan(sum, s_total);
     for (int b = b0; b < b1; ++b)
     {
         *RPPB_WR(prefix + b) = run;
@@ -138,12 +145,13 @@ __global__ void __launch_bounds__(1024) ragged_prefix_kernel(Count count, int n,
     if (t == threads - 1) *RPPB_WR(prefix + n) = run;
 }
 
+inline int ragged_prefix_threads(int n) { return std::min(1024, std::max(1, (n + 31) / 32) * 32); }
+
 template <class Count>
 inline void launch_ragged_prefix(Count count, int n, long long* prefix, cudaStream_t s, unsigned* zero = nullptr,
                                  int zeroWords = 0)
 {
-    const int threads = std::min(1024, std::max(1, (n + 31) / 32) * 32);
-    ragged_prefix_kernel<Count><<<1, threads, 0, s>>>(count, n, prefix, zero, zeroWords);
+    ragged_prefix_kernel<Count><<<1, ragged_prefix_threads(n), 0, s>>>(count, n, prefix, zero, zeroWords);
     count_launch(1);
 }
 

@@ -324,6 +324,11 @@ __global__ void __launch_bounds__(kThreads, 4)
                     float outRateAll)
 {
     extern __shared__ float s_lut[];   // the table, then (down-mixing) each compute warp's staged slice span
+    __shared__ long long s_prefix[kPrefixCache];
+    grid_dependency_wait();   // the prefix, when launched after the held-weights kernel
+    prefix = cache_prefix(dependency_result(prefix), n, s_prefix);   // ends with __syncthreads
+    const long long total = prefix[n];
+    if (total == 0) return;
     const int pairCount = kPairs ? int(resample_pair_entries(wd.lutSize, wd.padLeft, wd.padRight)) : 0;
     float* s_spans = s_lut + (kPairs ? 2 * pairCount : ((wd.lutSize + 3) & ~3));
     __shared__ __align__(16) float s_phase[2][kGroup][kBlock];
@@ -343,9 +348,6 @@ __global__ void __launch_bounds__(kThreads, 4)
                                                                           (kPairs ? wd.padLeft : 0))) -
                                             0x5A000000u};   // 8 * 0x4B400000 mod 2^32
     const int lobes = wd.lobes;
-    __shared__ long long s_prefix[kPrefixCache];
-    prefix = cache_prefix(prefix, n, s_prefix);   // ends with __syncthreads
-    const long long total = prefix[n];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     // the CTA's unit j of group g
@@ -531,7 +533,9 @@ constexpr int kHeldLobes = 16;
 constexpr int kItemBlocks = 16;      // blocks of an item
 constexpr int kHeldCtas = 2;         // per SM
 constexpr int kHeldSpan = 1024;      // staged samples of a block: ratios up to 3.8
-constexpr int kHeldPeriod = 64;      // longer periods share nothing: items of one block
+constexpr int kHeldPeriod = 64;      // longest period between blocks that share weights
+constexpr int kHeldShare = 4;        // blocks of a sample that share weights, at least
+constexpr int kHeldMono = 16, kHeldMixed = 32;   // and its blocks: the first and the last are summed output by output
 constexpr int kHeldWarps = 8;        // compute warps: 8 outputs per pass and warp, four passes per block
 constexpr int kHeldCompute = kHeldWarps * 32, kHeldThreads = kHeldCompute + 32;
 constexpr int kHeldOuts = kBlock / (kHeldWarps * 8);   // outputs per thread
@@ -555,45 +559,120 @@ __device__ __forceinline__ int phase_period(float inRate, float outRate)
     return p <= kHeldPeriod ? p : 0;
 }
 
-// How a resampled sample's blocks are dealt to items: item i takes blocks i % period + period * (first + j).
+// Whether the held-weights kernel takes a sample: its rates repeat a phase (48 to 44.1 kHz or 16 to 44.1 kHz, with
+// items of one block, took 1230 and 1209 us there and 429 and 380 us in resample_kernel on 64 clips of 8 s), the span of
+// a block fits the staging (96 to 16 kHz, every block output by output: stereo 1193 against 319 us), and it has enough
+// blocks (4096 stereo clips of 16 blocks 498 against 413 us, 2048 of 32 blocks 368 against 409; mono 247 against 282
+// and 218 against 273).
+__device__ __forceinline__ bool held_sample(int outEnd, int period, float inRate, float outRate, bool mix)
+{
+    if (period == 0 || float(kBlock) * inRate > float(kHeldSpan - 2 * kHeldLobes - 4) * outRate) return false;
+    return (outEnd + kBlock - 1) / kBlock >= max(kHeldShare * period, mix ? kHeldMixed : kHeldMono);
+}
+
+// How its blocks are dealt to items: item i takes blocks i % period + period * (first + j).
 struct ItemPlan
 {
     int blocks, period, per, groups;
-    __device__ __forceinline__ ItemPlan(int outEnd, float inRate, float outRate)
+    __device__ __forceinline__ ItemPlan(int outEnd, int phasePeriod)
     {
         blocks = (outEnd + kBlock - 1) / kBlock;
-        const int p = phase_period(inRate, outRate);
-        period = p == 0 ? 1 : max(1, min(p, blocks));
+        period = phasePeriod;
         const int each = (blocks + period - 1) / period;
-        groups = p == 0 ? each : (each + kItemBlocks - 1) / kItemBlocks;
-        per = groups > 0 ? (each + groups - 1) / groups : 0;
+        groups = (each + kItemBlocks - 1) / kItemBlocks;
+        per = (each + groups - 1) / groups;
     }
     __device__ __forceinline__ long long items() const { return (long long)period * groups; }
 };
 
-struct HeldCount
+// Deals the samples to the two kernels: held[0..n] and general[0..n] are the prefixes of their work units.  The
+// held-weights kernel takes what held_sample admits when the batch has minBlocks such blocks, else nothing.
+__global__ void __launch_bounds__(1024) resample_split_kernel(const float* __restrict__ inRateT,
+                                                              const float* __restrict__ outRateT,
+                                                              const int* __restrict__ dims, bool mix, int n,
+                                                              int minBlocks, long long* __restrict__ held,
+                                                              long long* __restrict__ general,
+                                                              unsigned long long* __restrict__ nextItem)
 {
-    const float* inRate;
-    const float* outRate;
-    const int* dims;
-    bool mix;
-    __device__ long long operator()(int b) const
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    struct Units
     {
-        const int L = *RPPB_RD(dims + 2 * b), Cs = *RPPB_RD(dims + (2 * b + 1));
-        const float ir = *RPPB_RD(inRate + b), orr = *RPPB_RD(outRate + b);
-        if (L <= 0 || Cs <= 0) return 0;
-        if (ir == orr) return ((long long)L * (mix ? 1 : Cs) + kCopyChunk - 1) / kCopyChunk;
+        long long all;     // of the general kernel
+        int items, blocks; // of the held-weights kernel (0: not for it)
+        bool copy;         // equal rates: either kernel
+    };
+    auto units = [&](int b) {
+        Units u{0, 0, 0, false};
+        const int L = *RPPB_RD(dims + 2 * b), Cs = *RPPB_RD(dims + (2 * b + 1)), C = mix ? 1 : Cs;
+        const float ir = *RPPB_RD(inRateT + b), orr = *RPPB_RD(outRateT + b);
+        if (L <= 0 || Cs <= 0) return u;
+        u.copy = ir == orr;
+        if (u.copy)
+        {
+            u.all = ((long long)L * C + kCopyChunk - 1) / kCopyChunk;
+            return u;
+        }
         const int outEnd = out_length(L, ir, orr);
-        return outEnd <= 0 ? 0 : ItemPlan(outEnd, ir, orr).items();
+        if (outEnd <= 0) return u;
+        u.all = (outEnd + kBlock - 1) / kBlock;
+        const int period = phase_period(ir, orr);
+        if (C != 1 || Cs > 64 || !held_sample(outEnd, period, ir, orr, mix)) return u;
+        u.blocks = int(u.all);
+        u.items = int(ItemPlan(outEnd, period).items());
+        return u;
+    };
+    __shared__ long long s_total[2][32];
+    __shared__ int s_blocks;
+    const int t = threadIdx.x, threads = blockDim.x;
+    const int per = (n + threads - 1) / threads;
+    const int b0 = min(n, t * per), b1 = min(n, b0 + per);
+    if (t == 0)
+    {
+        s_blocks = 0;
+        *RPPB_WR(nextItem) = 0ull;
     }
-};
+    __syncthreads();
+    Units first{0, 0, 0, false};
+    int blocks = 0;                           // only whether the sum reaches minBlocks counts
+    long long all = 0, items = 0, rest = 0;   // the general kernel's units alone; both kernels' units when both run
+    for (int b = b0; b < b1; ++b)
+    {
+        const Units u = units(b);
+        if (b == b0) first = u;
+        blocks = min(blocks + min(u.blocks, minBlocks), minBlocks);
+        all += u.all;
+        items += u.copy ? u.all : (long long)u.items;
+        rest += u.copy || u.items > 0 ? 0 : u.all;
+    }
+    blocks = __reduce_add_sync(0xffffffffu, blocks);
+    if ((t & 31) == 0 && blocks > 0) atomicAdd(&s_blocks, blocks);
+    __syncthreads();
+    const bool use = s_blocks >= minBlocks;
+    long long h = use ? items : 0, g = use ? rest : all;
+    h = block_exclusive_scan(h, s_total[0]);
+    g = block_exclusive_scan(g, s_total[1]);
+    for (int b = b0; b < b1; ++b)
+    {
+        const Units u = b == b0 ? first : units(b);
+        *RPPB_WR(held + b) = h;
+        *RPPB_WR(general + b) = g;
+        const bool mine = use && (u.copy || u.items > 0);
+        h += !mine ? 0 : u.copy ? u.all : (long long)u.items;
+        g += mine ? 0 : u.all;
+    }
+    if (t == threads - 1)
+    {
+        *RPPB_WR(held + n) = h;
+        *RPPB_WR(general + n) = g;
+    }
+}
 
 constexpr int kBlockHeld = 0, kBlockEdge = 1, kBlockOther = 2;
 struct HeldItem
 {
     const float* x;
     float* y;
-    int L, Csrc, C, unit;      // unit: copies only
+    int L, Csrc, unit;         // unit: copies only
     int mode;                  // kUnitSkip, kUnitCopy or kUnitResample; -1: no item left
     int count, held;           // blocks; the first `held` of them share the item's weights
     int lo, span;              // the blocks' samples are [origin + lo, origin + lo + span)
@@ -642,23 +721,18 @@ __device__ RPPB_OUT_OF_LINE void other_blocks(const Win<true, true, true>& win, 
         const int k = threadIdx.x;
         if (k >= it.outs[e]) continue;
         const float p = phase[k];
-        const int origin = it.origin[e], L = it.L, C = it.C;
+        const int origin = it.origin[e], L = it.L;
         const int xc = int(ceilf(p));
         int loc0 = xc - kHeldLobes, loc1 = xc + kHeldLobes;
         if (loc0 + origin < 0) loc0 = -origin;
         if (loc1 + origin > L) loc1 = L - origin;
         const long long outPos = (long long)it.block[e] * kBlock + k;
-        if (kMix || C == 1)
-        {
-            auto at = [&](int l) {
-                return kMix ? mix((long long)origin + l) : __ldg(RPPB_RD(it.x + ((long long)origin + l)));
-            };
-            const int ex = int((__float_as_uint(p) >> 23) & 0xffu) - 127;
-            *RPPB_WR(it.y + outPos) = ex >= exactMinE && ex <= exactMaxE ? mono_taps_exact(win, at, loc0, loc1, p)
-                                                                         : mono_taps(win, at, loc0, loc1, p);
-        }
-        else
-            channel_taps(win, it.x + (long long)origin * C, it.y + outPos * C, C, loc0, loc1, p);
+        auto at = [&](int l) {
+            return kMix ? mix((long long)origin + l) : __ldg(RPPB_RD(it.x + ((long long)origin + l)));
+        };
+        const int ex = int((__float_as_uint(p) >> 23) & 0xffu) - 127;
+        *RPPB_WR(it.y + outPos) = ex >= exactMinE && ex <= exactMaxE ? mono_taps_exact(win, at, loc0, loc1, p)
+                                                                     : mono_taps(win, at, loc0, loc1, p);
     }
 }
 
@@ -669,6 +743,7 @@ __global__ void __launch_bounds__(kHeldThreads, 2)
                          const int* __restrict__ dims, ResampleWindowDev wd, bool normalize,
                          const long long* __restrict__ prefix, unsigned long long* __restrict__ nextItem, int n)
 {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     extern __shared__ float s_lut[];   // the padded (value, next - value) table, then two staged spans
     const int pairCount = int(resample_pair_entries(wd.lutSize, wd.padLeft, wd.padRight));
     float* s_span = s_lut + 2 * pairCount;
@@ -704,25 +779,24 @@ __global__ void __launch_bounds__(kHeldThreads, 2)
         }
         const int b = ragged_find(prefix, n, w);
         const int local = int(w - prefix[b]);
-        const int L = *RPPB_RD(dims + 2 * b), Csrc = *RPPB_RD(dims + (2 * b + 1)), C = kMix ? 1 : Csrc;
+        const int L = *RPPB_RD(dims + 2 * b), Csrc = *RPPB_RD(dims + (2 * b + 1));
         const float inRate = *RPPB_RD(inRateT + b), outRate = *RPPB_RD(outRateT + b);
         const float* x = src + size_t(b) * srcStride;
-        const int mode = inRate == outRate ? kUnitCopy : (kMix && Csrc > 64) ? kUnitSkip : kUnitResample;
+        const int mode = inRate == outRate ? kUnitCopy : kUnitResample;
         if (lane == 0)
         {
             it.x = x;
             it.y = dst + size_t(b) * dstStride;
             it.L = L;
             it.Csrc = Csrc;
-            it.C = C;
             it.unit = local;
             it.mode = mode;
             it.wc = kMix ? MonoMix::weight(max(Csrc, 1), normalize) : 1.f;
         }
         if (mode != kUnitResample) return;
         const int outFull = out_length(L, inRate, outRate);
-        const int outEnd = min(outFull, int(dstStride / uint32_t(C)));
-        const ItemPlan plan(outFull, inRate, outRate);
+        const int outEnd = min(outFull, int(dstStride));
+        const ItemPlan plan(outFull, phase_period(inRate, outRate));
         const double scale = __ddiv_rn(double(inRate), double(outRate));
         const float fscale = __double2float_rn(scale);
         const int residue = local % plan.period, j0 = local / plan.period * plan.per;
@@ -745,7 +819,7 @@ __global__ void __launch_bounds__(kHeldThreads, 2)
             const long long from = (long long)origin + lo;
             const long long to = (long long)origin + int(ceilf(ph[outs - 1])) + kHeldLobes;
             const int kind = __float_as_uint(first) != __float_as_uint(held)              ? kBlockOther
-                             : from < 0 || to > L || span > kHeldSpan || (!kMix && C != 1) ? kBlockEdge
+                             : from < 0 || to > L || span > kHeldSpan                      ? kBlockEdge
                                                                                            : kBlockHeld;
             // the blocks that share the weights first
             const unsigned share = __ballot_sync(all, kind == kBlockHeld);
@@ -783,7 +857,7 @@ __global__ void __launch_bounds__(kHeldThreads, 2)
         {
             const MonoMix mix{it.x, kMix ? it.Csrc : 1, it.wc};
             const long long L = it.L;
-            const long long count = kMix ? min(L, (long long)dstStride) : min(L * it.C, (long long)min(srcStride, dstStride));
+            const long long count = kMix ? min(L, (long long)dstStride) : min(L * it.Csrc, (long long)min(srcStride, dstStride));
             const long long i0 = (long long)it.unit * kCopyChunk, end = min(count, i0 + kCopyChunk);
             const float* x = it.x;
             float* y = it.y;
@@ -930,7 +1004,7 @@ __global__ void __launch_bounds__(kHeldThreads, 2)
 namespace {
 
 // The held-weights kernel serves windows of 16 lobes with a power-of-two table scale (what kaiser_sinc and the
-// reference's own window give at 16 lobes), whatever the rates; other windows take resample_kernel.
+// reference's own window give at 16 lobes) and the samples of held_sample; the rest take resample_kernel.
 bool resample_held_ok(const ResampleWindowDev& w, bool magic, bool fma)
 {
     return magic && fma && w.lobes == kHeldLobes &&
@@ -938,21 +1012,20 @@ bool resample_held_ok(const ResampleWindowDev& w, bool magic, bool fma)
 }
 
 template <bool kMix>
-void launch_held(Handle& h, void* scratch, const float* src, uint32_t srcStride, float* dst, uint32_t dstStride, int n,
+void launch_held(Handle& h, const float* src, uint32_t srcStride, float* dst, uint32_t dstStride, int n,
                  const float* inRate, const float* outRate, const int* dims, const ResampleWindowDev& w,
-                 bool normalize)
+                 bool normalize, int minBlocks, long long* held, long long* general, unsigned long long* next)
 {
     const size_t smem = resample_smem_floats(w, true, true) * sizeof(float);   // the table and two spans
     static_assert(kWarps * 256 == 2 * kHeldSpan, "resample_smem_floats counts the spans");
     const int grid = persistent_grid(h, reinterpret_cast<const void*>(resample_held_kernel<kMix>), kHeldThreads, smem);
-    Carver cv(scratch);
-    long long* prefix = cv.take<long long>(n + 1);
-    unsigned long long* next = cv.take<unsigned long long>(1);
-    launch_ragged_prefix(HeldCount{inRate, outRate, dims, kMix}, n, prefix, h.stream(),
-                         reinterpret_cast<unsigned*>(next), 2);
+    resample_split_kernel<<<1, ragged_prefix_threads(n), 0, h.stream()>>>(inRate, outRate, dims, kMix, n, minBlocks, held,
+                                                                          general, next);
+    count_launch();
+    check_cuda(cudaGetLastError(), "resample_split_kernel");
     launch_dependent(resample_held_kernel<kMix>, dim3(grid), dim3(kHeldThreads), smem, h.stream(),
                      "resample_held_kernel", src, srcStride, dst, dstStride, inRate, outRate, dims, w, normalize,
-                     static_cast<const long long*>(prefix), next, n);
+                     static_cast<const long long*>(held), next, n);
     count_launch();
 }
 
@@ -961,6 +1034,7 @@ void launch_held(Handle& h, void* scratch, const float* src, uint32_t srcStride,
 size_t resample_scratch_bytes(int n)
 {
     Carver cv(nullptr);
+    cv.take<long long>(n + 1);
     cv.take<long long>(n + 1);
     cv.take<unsigned long long>(1);
     return cv.used();
@@ -971,7 +1045,10 @@ void launch_resample(Handle& h, void* scratch, const float* src, uint32_t srcStr
                      int channels, bool downmix, bool normalize)
 {
     if (n <= 0) return;
-    long long* prefix = static_cast<long long*>(scratch);
+    Carver cv(scratch);
+    long long* prefix = cv.take<long long>(n + 1);
+    long long* heldPrefix = cv.take<long long>(n + 1);
+    unsigned long long* next = cv.take<unsigned long long>(1);
     ResampleWindowDev w = win;
     resample_pads(w);
     const bool pairs = w.padLeft >= 0 && resample_smem_floats(w, true, downmix) * sizeof(float) <= kPairTableLimit;
@@ -979,24 +1056,30 @@ void launch_resample(Handle& h, void* scratch, const float* src, uint32_t srcStr
     const bool magic = resample_magic_ok(w, pairs);
     const bool fma = resample_scale_pow2(w);
     resample_exact_range(w, magic, fma);
-    // The held-weights kernel pays from four full items per CTA on, by the batch's padded size: at 2 CTAs per SM
-    // 18944 blocks, 5 minutes at 16 kHz (clips of 3 s, mono / stereo: 32 clips 32 against 33 us and 45 against 38,
-    // 64 clips 43 against 52 us and 61 against 62, and 64 clips of 6 s 73 against 112 us).
+    // The held-weights kernel pays from two full items per CTA on, 9472 blocks at 2 CTAs per SM, 2.5 minutes at 16 kHz
+    // (against resample_kernel, mono / stereo from 44.1 kHz: 8 clips of 10 s 42 and 48, 56 and 54 us; 16 clips 56 and
+    // 81, 69 and 95 us; from 48 kHz 41 and 34, 48 and 48; 50 and 56, 68 and 83 us).  resample_split_kernel counts them;
+    // it and the second kernel cost 2 us, so batches that are below twice that when padded skip both.
     const long long padded = (long long)n * ((dstStride + kBlock - 1) / kBlock);
-    const bool many = padded >= 4ll * kItemBlocks * kHeldCtas * h.num_sms();
-    if (many && (downmix || channels <= 1) && resample_held_ok(w, magic, fma))
+    const int minBlocks = 2 * kItemBlocks * kHeldCtas * h.num_sms();
+    const bool split = padded >= 2ll * minBlocks && (downmix || channels <= 1) && resample_held_ok(w, magic, fma);
+    if (split)
     {
-        if (downmix)
-            launch_held<true>(h, scratch, src, srcStride, dst, dstStride, n, inRate, outRate, dims, w, normalize);
-        else
-            launch_held<false>(h, scratch, src, srcStride, dst, dstStride, n, inRate, outRate, dims, w, normalize);
-        return;
+        auto held = downmix ? launch_held<true> : launch_held<false>;
+        held(h, src, srcStride, dst, dstStride, n, inRate, outRate, dims, w, normalize, minBlocks, heldPrefix, prefix, next);
     }
-    launch_ragged_prefix(ResampleCount{inRate, outRate, dims, downmix, nullptr, 0.f}, n, prefix, h.stream());
+    else
+        launch_ragged_prefix(ResampleCount{inRate, outRate, dims, downmix, nullptr, 0.f}, n, prefix, h.stream());
     auto go = [&](auto kernel) {
         const int grid = persistent_grid(h, reinterpret_cast<const void*>(kernel), kThreads, smem);
-        kernel<<<grid, kThreads, smem, h.stream()>>>(src, srcStride, dst, dstStride, inRate, outRate, dims, w,
-                                                     normalize, prefix, n, nullptr, 0.f);
+        const long long* units = prefix;
+        const RppbClip* clips = nullptr;
+        if (split)   // starts while the held-weights kernel ends
+            launch_dependent(kernel, dim3(grid), dim3(kThreads), smem, h.stream(), "resample_kernel", src, srcStride, dst,
+                             dstStride, inRate, outRate, dims, w, normalize, units, n, clips, 0.f);
+        else
+            kernel<<<grid, kThreads, smem, h.stream()>>>(src, srcStride, dst, dstStride, inRate, outRate, dims, w,
+                                                         normalize, units, n, clips, 0.f);
     };
     if (downmix && magic && fma) go(resample_kernel<true, false, true, true, true>);
     else if (downmix && magic) go(resample_kernel<true, false, true, true>);

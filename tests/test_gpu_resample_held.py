@@ -1,51 +1,127 @@
-"""resample with 16-lobe windows: the kernel that holds a block's weights across the blocks that share them.  Bit
-for bit the oracle's samples at the edges of its rule: rates with short, long and no phase period, ratios whose
-span does and does not fit, clips that end around a block or an item, odd row widths, down-mixed channels."""
+"""resample with 16-lobe windows on large batches, where a kernel that holds a block's weights across the blocks that
+share them takes the samples that have enough of them and the general kernel the rest.  Bit for bit the oracle's
+samples at the edges of its rule: rates with short, long and no phase period, ratios whose span does and does not fit,
+clips that end around a block or an item, odd row widths, down-mixed channels, rows too narrow for the clips; and both
+kernels' times on rates that share nothing."""
 import numpy as np
 import pytest
 
 torch = pytest.importorskip("torch")
 
 from gpu_util import canvas, dev, host  # noqa: E402
-from rpp_b200 import audio  # noqa: E402
+from rpp_b200 import audio, lib  # noqa: E402
 from rpp_b200.types import audio_desc  # noqa: E402
 from rpp_b200.windows import kaiser_sinc  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("channels", [1, 2, 3])
-@pytest.mark.parametrize("rates", [(48000, 16000), (44100, 16000), (22050, 16000), (32000, 16000), (8000, 16000),
-                                   (16000, 22050), (16000, 48000), (96000, 16000), (44100.5, 16000), (61440, 16000)])
-def test_held_weights_equal_oracle(gpu, oracle, rates, channels):
-    r = np.random.default_rng(int(rates[0]) + channels)
+SHARED = [(48000, 16000), (44100, 16000), (22050, 16000), (32000, 16000), (8000, 16000), (16000, 48000),
+          (16000, 24000), (61440, 16000)]
+OTHER = [(16000, 22050), (96000, 16000), (44100.5, 16000)]   # long period, span too long, no period
+OUTS = [1, 257, 16 * 256 + 1, 32 * 256 + 1, 5 * 256 * 16 + 7, 29999, 115 * 256, 30000]
+
+
+def held_blocks_needed():
+    """Blocks from which the held-weights kernel is used: two items of 16 for each of its CTAs, 2 per SM."""
+    return 64 * torch.cuda.get_device_properties(0).multi_processor_count
+
+
+def setup(rates, channels, seed, reps, outs=OUTS):
+    """(reps copies of the clips of `outs` outputs: descriptor and tensors, oracle samples of one copy)."""
+    r = np.random.default_rng(seed)
     ratio = rates[0] / rates[1]
-    outs = [1, 255, 256, 257, 1279, 1281, 5 * 256 * 3 + 7, 30000]
     lens = np.array([max(1, int(o * ratio)) for o in outs], np.int32)
     n, L = len(lens), int(lens.max()) + 1   # rows of odd and even width over the rates
     x = r.normal(0, 0.3, (n, L * channels)).astype(np.float32)
-    lut, scale, center, lobes = kaiser_sinc(16)
-    ir, orr = np.full(n, rates[0], np.float32), np.full(n, rates[1], np.float32)
     width = int(np.ceil(L / ratio)) + 9
-    ones = np.stack([lens, np.ones(n, np.int32)], 1).astype(np.int32)
+    tile = lambda a: dev(a).repeat(reps, *[1] * (a.ndim - 1))   # noqa: E731
     dims = np.stack([lens, np.full(n, channels, np.int32)], 1).astype(np.int32)
+    s = dict(x=tile(x), dims=tile(dims), ir=torch.full((n * reps,), float(rates[0]), device="cuda"),
+             orr=torch.full((n * reps,), float(rates[1]), device="cuda"), n=n * reps, L=L, width=width,
+             channels=channels)
+    return s, x, lens
+
+
+def call(gpu, s, out, width):
+    lut, scale, center, lobes = kaiser_sinc(16)
+    s.setdefault("lut", dev(lut))
+    ch = s["channels"]
+    sd, od = audio_desc(s["n"], s["L"], channels=ch, num_dims=3 if ch > 1 else 2), audio_desc(s["n"], width)
+    if ch > 1:
+        return audio.downmix_resample(s["x"], sd, out, od, s["ir"], s["orr"], s["dims"], False, s["lut"], scale, center,
+                                      lobes, gpu)
+    return audio.resample(s["x"], sd, out, od, s["ir"], s["orr"], s["dims"],
+                          audio.resampling_window(s["lut"], scale, center, lobes), gpu)
+
+
+@pytest.mark.parametrize("channels", [1, 2, 3])
+@pytest.mark.parametrize("rates", SHARED + OTHER)
+def test_large_batches_equal_oracle(gpu, oracle, rates, channels):
+    full = sum(-(-o // 256) for o in OUTS if o > 100 * 256)   # blocks of one copy that every period admits
+    reps = -(-held_blocks_needed() * 21 // (20 * full))
+    s, x, lens = setup(rates, channels, int(rates[0]) + channels, reps)
+    assert s["n"] * -(-s["width"] // 256) >= 2 * held_blocks_needed()   # the padded size admits the kernel too
+    n, L, width = len(lens), s["L"], s["width"]
     mono = x
     if channels > 1:
         mono = np.zeros((n, L), np.float32)
-        oracle.down_mixing(x, mono, dims.ravel(), False)
+        oracle.down_mixing(x, mono, np.stack([lens, np.full(n, channels, np.int32)], 1).astype(np.int32).ravel(), False)
+    lut, scale, center, lobes = kaiser_sinc(16)
     ref = np.full((n, width), -12345.0, np.float32)
-    oracle.resample(mono, ref, ir, orr, ones.ravel(), lut, scale, center, lobes)
-    lut_d, xd, sd = dev(lut), dev(x), audio_desc(n, L, channels=channels, num_dims=3 if channels > 1 else 2)
+    oracle.resample(mono, ref, np.full(n, rates[0], np.float32), np.full(n, rates[1], np.float32),
+                    np.stack([lens, np.ones(n, np.int32)], 1).astype(np.int32).ravel(), lut, scale, center, lobes)
+    for w in (width, 28673):   # the second is too narrow for the longer clips, by a block and a part of one
+        out = canvas((s["n"], w))
+        launches = lib.load().rppbGetLaunchCount()
+        assert call(gpu, s, out, w) == 0
+        assert lib.load().rppbGetLaunchCount() - launches == 3   # the work lists and both kernels
+        torch.cuda.synchronize()
+        same = (out.view(reps, n, w).view(torch.int32) == dev(np.ascontiguousarray(ref[:, :w])).view(torch.int32)).all()
+        assert bool(same)
 
-    def call(w):
-        out = canvas((n, w))
-        if channels > 1:
-            assert audio.downmix_resample(xd, sd, out, audio_desc(n, w), dev(ir), dev(orr), dev(dims), False, lut_d,
-                                          scale, center, lobes, gpu) == 0
-        else:
-            win = audio.resampling_window(lut_d, scale, center, lobes)
-            assert audio.resample(xd, sd, out, audio_desc(n, w), dev(ir), dev(orr), dev(dims), win, gpu) == 0
-        return host(out)
 
-    np.testing.assert_array_equal(call(width), ref)
-    np.testing.assert_array_equal(call(1000), ref[:, :1000])   # rows too narrow for the longer clips
+@pytest.mark.parametrize("rates", [(48000, 16000), (44100, 16000)])
+def test_mixed_batch_equals_oracle(gpu, oracle, rates):
+    """Samples for either kernel, equal-rate copies, empty samples and rates that change from row to row."""
+    reps = -(-held_blocks_needed() * 21 // (20 * 3 * 115))
+    kinds = [(rates[0], 29999), (16000, 30000), (96000, 30000), (rates[0], 29500), (44100.5, 20000), (rates[0], 0),
+             (rates[0], 29441), (22050, 700), (16000, 0)]
+    ir = np.array([k[0] for k in kinds], np.float32)
+    lens = np.array([int(k[1] * k[0] / 16000) for k in kinds], np.int32)
+    n, L, width = len(kinds), int(lens.max()) + 3, 30009
+    r = np.random.default_rng(7)
+    x = r.normal(0, 0.3, (n, L)).astype(np.float32)
+    dims = np.stack([lens, np.ones(n, np.int32)], 1).astype(np.int32)
+    lut, scale, center, lobes = kaiser_sinc(16)
+    ref = np.full((n, width), -12345.0, np.float32)
+    oracle.resample(x, ref, ir, np.full(n, 16000, np.float32), dims.ravel(), lut, scale, center, lobes)
+    s = dict(x=dev(x).repeat(reps, 1), dims=dev(dims).repeat(reps, 1), ir=dev(ir).repeat(reps),
+             orr=torch.full((n * reps,), 16000.0, device="cuda"), n=n * reps, L=L, channels=1)
+    out = canvas((n * reps, width))
+    assert call(gpu, s, out, width) == 0
+    torch.cuda.synchronize()
+    assert bool((out.view(reps, n, width).view(torch.int32) == dev(ref).view(torch.int32)).all())
+
+
+@pytest.mark.parametrize("rates,channels", [((48000, 44100), 1), ((16000, 44100), 2), ((96000, 16000), 2)])
+def test_rates_that_share_no_weights_keep_their_time(gpu, rates, channels):
+    """One large batch against its four quarters, which are too small for the held-weights kernel: with that kernel on
+    such rates the batch takes 2.5 times its quarters or more."""
+    s, _, _ = setup(rates, channels, 3, 24, outs=[110000, 109000])
+    q = dict(s, n=s["n"] // 4, x=s["x"][:s["n"] // 4], dims=s["dims"][:s["n"] // 4])
+    assert s["n"] * -(-s["width"] // 256) >= 2 * held_blocks_needed() > q["n"] * -(-s["width"] // 256)
+
+    def best(v):
+        out = canvas((v["n"], v["width"]))
+        times = []
+        for _ in range(8):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            assert call(gpu, v, out, v["width"]) == 0
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times)
+
+    assert best(s) < 1.5 * 4 * best(q)
