@@ -1422,11 +1422,14 @@ extern "C" SHARED_PUBLIC RppStatus rppt_normalize_gpu(RppPtr_t srcPtr, RpptGener
         const int compute = computeMeanStddev & 3;
         // both statistics per contiguous row: one kernel, no task list
         void *meanDirect = nullptr, *stdDirect = nullptr;
-        const bool rowwise = axisMask == 2 && compute == 3 && sd.strides[2] == 1 &&
+        bool rowwise = axisMask == 2 && compute == 3 && sd.strides[2] == 1 &&
                              normalize_rows_fit(int(std::min<uint32_t>(sd.dims[2], INT32_MAX))) &&
                              h.device_writable(meanTensor, &meanDirect) && h.device_writable(stdDevTensor, &stdDirect);
         // roi lengths are needed on the host (parameter counts, work list)
         const std::vector<uint32_t> roi = roi_to_host(h, roiTensor, size_t(n) * 4);
+        // that kernel goes by the destination's rows; roi rows past them have statistics all the same
+        const uint64_t dstRows = dd.strides[1] ? (uint64_t(dd.strides[0]) + dd.strides[1] - 1) / dd.strides[1] : 0;
+        for (int b = 0; b < n && rowwise; ++b) rowwise = std::min(roi[4 * b + 2], sd.dims[1]) <= dstRows;
         int maxSize = 1, maxCount = 0;
         std::vector<NormalizeSample> samples(n);
         std::vector<int4> tasks;

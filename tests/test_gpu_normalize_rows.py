@@ -39,3 +39,22 @@ def test_rows_equal_oracle(gpu, oracle, cols):
         a = dev(src)
         assert audio.normalize(a, d, a, d, 2, dev(mean), dev(std), 3, 1.5, 0.25, roi.ravel(), gpu) == 0
         np.testing.assert_array_equal(host(a), host(out))
+
+
+def test_rows_past_the_destination_have_statistics(gpu, oracle):
+    """A destination of fewer rows than the roi: its rows normalized, every roi row's statistics written."""
+    r = np.random.default_rng(3)
+    n, R, kept, cols = 3, 11, 7, 130
+    src = (r.standard_normal((n, R, cols)) * 3 + 1).astype(np.float32)
+    roi = np.zeros((n, 4), np.uint32)
+    roi[:, 2], roi[:, 3] = R, cols
+    m_ref, s_ref = np.zeros(n * R, np.float32), np.zeros(n * R, np.float32)
+    exp = np.zeros((n, R, cols), np.float32)
+    oracle.normalize_2d(src, exp, 2, m_ref, s_ref, 3, 1.0, 0.0, roi.ravel())
+    out = torch.full((n, kept, cols), 7.0, device="cuda")
+    m, s = torch.full((n * R,), 5.0, device="cuda"), torch.full((n * R,), 5.0, device="cuda")
+    assert audio.normalize(dev(src), generic_desc((n, R, cols)), out, generic_desc((n, kept, cols)), 2, m, s, 3, 1.0,
+                           0.0, roi.ravel(), gpu) == 0
+    np.testing.assert_array_equal(host(m), m_ref)
+    np.testing.assert_allclose(host(s), s_ref, rtol=1e-6, atol=0)
+    np.testing.assert_allclose(host(out), exp[:, :kept], rtol=1e-5, atol=1e-5)
