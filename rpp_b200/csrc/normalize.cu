@@ -335,7 +335,9 @@ void launch_normalize_rows(Handle& h, const NormalizeArgs& a, int maxCount)
 {
     if (a.n <= 0 || a.dstStride0 == 0) return;
     const int rowsPerSample = int((a.dstStride0 + a.dstStride1 - 1) / a.dstStride1);
-    const int stage = std::max(maxCount, 1) | 1;   // odd: the warps' rows start in different banks
+    // by steps of 128, so that ragged batches share 32 entries of persistent_grid's cache; odd: the warps' rows start in
+    // different banks
+    const int stage = ((std::max(maxCount, 1) + 127) & ~127) | 1;
     const size_t smem = size_t(kThreads / 32) * stage * sizeof(float);
     const long long rows = (long long)a.n * rowsPerSample;
     const int grid = int(std::min<long long>((rows + kThreads / 32 - 1) / (kThreads / 32),
