@@ -133,8 +133,12 @@ def dist_init():
 def run_reference(args, world, rank):
     if rank != 0:
         return
-    from oracle import Reference
+    from oracle import Reference, build_reference
     from rpp_b200.types import RpptImagePatch
+    if not build_reference():
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's host library is not built and its "
+                          "sources are absent (oracle/build_ref.sh)"}), flush=True)
+        return
     threads = os.cpu_count() or 1
     ref = Reference(threads=threads)
     x, lens = synth.gapped_clips(n=args.clips)
