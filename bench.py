@@ -128,6 +128,20 @@ def dist_init():
     return replicas.env()
 
 
+def rounded(v):
+    """`v` with every float in it to five significant digits."""
+    if isinstance(v, dict):
+        return {k: rounded(x) for k, x in v.items()}
+    if isinstance(v, (list, tuple)):
+        return [rounded(x) for x in v]
+    return float(f"{v:.5g}") if isinstance(v, float) else v
+
+
+def without(v, key):
+    """`v` less every entry named `key` in it."""
+    return {k: without(x, key) for k, x in v.items() if k != key} if isinstance(v, dict) else v
+
+
 # ---------------------------------------------------------------- the reference arm
 
 def run_reference(args, world, rank):
@@ -1094,6 +1108,13 @@ def run_b200(args, world, rank, local):
             "gpu_launches": int(launches),
             "clocks": clocks,
         }
+        # The line stays below 13 KB (a reader of limited length cut it at 21): the measurements' digits beyond the
+        # fifth are left out, and the precision study's breakdown by dynamic range goes to stderr.
+        for key in ("precision", "multirate", "serving", "err_vs_fp64", "nsr", "tensor_core_engine"):
+            line[key] = rounded(line[key])
+        if precision and "nfft" in precision:
+            print(json.dumps({"precision": line["precision"]}), file=sys.stderr, flush=True)
+            line["precision"] = without(line["precision"], "by_dynamic_range")
         print(json.dumps(line), flush=True)
     h.close()
     replicas.finish()
