@@ -96,7 +96,7 @@ __global__ void check_table_kernel(CheckTable t) { g_checkTable = t; }
 // The checked sources, for naming a violation's file from its site (common.cuh: RPPB_SITE).
 const char* const kCheckFiles[] = {"common.cuh", "preemph.cu", "downmix.cu", "downmix.cuh", "resample.cu",
                                    "spectrogram.cu", "stft.cuh", "stft_pair.cuh", "fft.cuh", "mel.cu",
-                                   "mel_sweep.cuh", "mel_tables.cuh", "to_decibels.cu", "nsr.cu", "fused.cu",
+                                   "mel_sweep.cuh", "mel_tables.cuh", "to_decibels.cu", "nsr.cu", "nsr_stored.cu", "fused.cu",
                                    "fused_queue.cuh", "fused_tc.cu", "tc_dft.cu", "tcgen05.cuh", "host_io.cu",
                                    "server.cu", "slice.cu", "normalize.cu", "normalize_nd.cu", "pcm.cu", "autotune.cu", "check.cu"};
 

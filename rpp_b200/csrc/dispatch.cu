@@ -240,7 +240,7 @@ extern "C" SHARED_PUBLIC RppStatus rppt_non_silent_region_detection_gpu(RppPtr_t
         const int n = int(srcDescPtr->n);
         if (n <= 0) return RPP_SUCCESS;
         const uint32_t stride = srcDescPtr->strides.nStride;
-        const size_t scratchBytes = nsr_scratch_bytes(n, stride, resetInterval);
+        const size_t scratchBytes = nsr_scratch_bytes(n, stride, windowLength, resetInterval);
         Carver m(nullptr);
         m.take<int>(n);
         m.take<int>(2 * n);

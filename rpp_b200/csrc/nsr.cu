@@ -15,7 +15,7 @@
 // replayed, in exactly the reference's order (add the new square, store sum * (1/windowLength), subtract
 // the square leaving the window; explicit round-to-nearest intrinsics, no FMA), and, if its exact values
 // lie inside the cutoff's interval too, the blocks that may hold the maximum.  Clips that this does not settle have
-// every block replayed.  Begin and length are therefore the host path's on every input.
+// every block replayed, and many short ones have from the start (nsr_stored.cu).  Begin and length are therefore the host path's on every input.
 //   1. energy_kernel: FP64 energies of 64-sample chunks, one streaming pass over the signal (HBM-bound: 30 us
 //      for 256 clips of 1 to 16 s, 4.6 TB/s);
 //   2. region_kernel: one CTA per sample: scan of the energies, cutoff interval, both ends, replays (15 to
@@ -984,10 +984,24 @@ size_t block_count(int n, uint32_t srcStride, int resetInterval)
     return resetInterval == -1 ? size_t(n) : size_t(n) * ((size_t(srcStride) + resetInterval - 1) / resetInterval);
 }
 
+// Many short samples: nsr_stored.cu's kernels.  On signals that end in silence, where intervals need a replay (window 512
+// up to 8000 samples a row, 2048 above; 35 % silence at the end), those against these took, us: 1024 samples of 1600 44 and
+// 65, of 8000 149 and 233, of 16000 210 and 200, of 32000 288 and 359, of 64000 439 and 347; 8192 of 8000 280 and 1238;
+// 512 of 8000 146 and 144, of 32000 253 and 187.  (Without silence intervals are faster from 4000 samples on, 8192 of
+// 16000 282 instead of 515 us.)
+bool stored(int n, uint32_t srcStride, int windowLength, int resetInterval)
+{
+    constexpr int kSamples = 1024;
+    constexpr long long kSteps = 49152;   // of a sample's chains: 32768 samples with a window of 2048
+    const long long blocks = resetInterval == -1 ? 1 : ((long long)srcStride + resetInterval - 1) / resetInterval;
+    return n >= kSamples && (long long)srcStride + blocks * windowLength <= kSteps;
+}
+
 }  // namespace
 
-size_t nsr_scratch_bytes(int n, uint32_t srcStride, int resetInterval)
+size_t nsr_scratch_bytes(int n, uint32_t srcStride, int windowLength, int resetInterval)
 {
+    if (stored(n, srcStride, windowLength, resetInterval)) return nsr_stored_scratch_bytes(n, srcStride, resetInterval);
     Carver cv(nullptr);
     cv.take<unsigned long long>(2);
     cv.take<double>(size_t(n) * energy_pitch(srcStride));
@@ -1001,6 +1015,7 @@ size_t nsr_scratch_bytes(int n, uint32_t srcStride, int resetInterval)
 void launch_nsr(Handle& h, void* scratch, const NsrArgs& a)
 {
     if (a.n <= 0) return;
+    if (stored(a.n, a.srcStride, a.windowLength, a.resetInterval)) return launch_nsr_stored(h, scratch, a);
     Carver cv(scratch);
     const long long pitch = energy_pitch(a.srcStride);
     ExactList list;

@@ -102,8 +102,12 @@ struct NsrArgs
     int resetInterval;
 };
 // Prefix energies of the samples' 64-sample chunks (FP64), the list of undecided samples and their reset blocks' maxima.
-size_t nsr_scratch_bytes(int n, uint32_t srcStride, int resetInterval);
+size_t nsr_scratch_bytes(int n, uint32_t srcStride, int windowLength, int resetInterval);
 void launch_nsr(Handle& h, void* scratch, const NsrArgs& a);
+// The same for many short samples (launch_nsr chooses): moving-mean-square buffer (srcStride floats per sample),
+// per-reset-block maxima and the prefix.
+size_t nsr_stored_scratch_bytes(int n, uint32_t srcStride, int resetInterval);
+void launch_nsr_stored(Handle& h, void* scratch, const NsrArgs& a);
 
 // Mel filter placement parameters (maxFreq already resolved: 0 -> sampleRate / 2).
 struct MelParams

@@ -107,6 +107,48 @@ def test_many_clips_with_every_block_replayed(gpu, oracle, reset, window, ref):
     np.testing.assert_array_equal(length, l_ref)
 
 
+@pytest.mark.parametrize("reset,window,top", [(8192, 2048, 9000), (8192, 512, 1500), (512, 300, 3000),
+                                               (-1, 2048, 9000), (8192, 100, 2000), (30, 40, 900), (8192, 9000, 3000)])
+@pytest.mark.parametrize("n", [1023, 1024, 1500])
+def test_many_short_clips(gpu, oracle, n, reset, window, top):
+    """Either side of the number of clips from which short ones have their moving mean squares stored."""
+    r = np.random.default_rng(14)
+    lens = r.integers(0, top + 1, n).astype(np.int32)
+    x = np.zeros((n, top + 3), np.float32)
+    for i, k in enumerate(lens):
+        x[i, k // 8:k - k // 3] = r.normal(0, 0.2, k - k // 3 - k // 8)
+    k = int(np.argmax(lens))
+    x[k, lens[k] // 2] = np.nan
+    x[k - 1, :] = np.where(np.arange(top + 3) == lens[k - 1] // 2, np.inf, x[k - 1])
+    with np.errstate(invalid="ignore"):
+        b_ref, l_ref = oracle.nsr(x, lens, -60.0, window, 0.0, reset)
+    begin, length, _ = detect(gpu, x, lens, window, reset)
+    np.testing.assert_array_equal(begin, b_ref)
+    np.testing.assert_array_equal(length, l_ref)
+
+
+def best_time(call):
+    times = []
+    for _ in range(7):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        call()
+        b.record()
+        b.synchronize()
+        times.append(a.elapsed_time(b))
+    return min(times)
+
+
+def test_many_short_clips_are_spread_over_the_gpu(gpu):
+    """16 times as many clips that end in silence, each replayed by a CTA of its own, take 10 times as long."""
+    r = np.random.default_rng(15)
+    lens = r.integers(2000, 4001, 8192).astype(np.int32)
+    x = r.normal(0, 0.1, (8192, 4000)).astype(np.float32)
+    x[np.arange(4000)[None] > lens[:, None] * 0.65] = 0.0
+    few, many = detect(gpu, x[:512], lens[:512], 512, 8192)[2], detect(gpu, x, lens, 512, 8192)[2]
+    assert best_time(many) < 5 * best_time(few)
+
+
 def test_replay_of_every_block_is_spread_over_the_gpu(gpu):
     """A long clip with a window just below the intervals' range: its 586 blocks replayed one after the other, a few
     at a time, take some hundred times the call with a window just inside."""
@@ -114,15 +156,6 @@ def test_replay_of_every_block_is_spread_over_the_gpu(gpu):
     lens = np.array([4800000], np.int32)
 
     def best(window):
-        call = detect(gpu, x, lens, window, 8192)[2]
-        times = []
-        for _ in range(7):
-            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-            a.record()
-            call()
-            b.record()
-            b.synchronize()
-            times.append(a.elapsed_time(b))
-        return min(times)
+        return best_time(detect(gpu, x, lens, window, 8192)[2])
 
     assert best(255) < 8 * best(256)
