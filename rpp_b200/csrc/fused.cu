@@ -44,8 +44,9 @@ __device__ __forceinline__ int thread_index()
     return t;
 }
 
-template <int NFFT, int TFX>
-__global__ void __launch_bounds__(kFusedThreads, (NFFT <= 512 ? 3 : 2)) frontend_kernel(FrontendArgs a, const float2* __restrict__ twiddle,
+// CTAS: resident CTAs per SM that the registers are sized for.
+template <int NFFT, int TFX, int CTAS>
+__global__ void __launch_bounds__(kFusedThreads, CTAS) frontend_kernel(FrontendArgs a, const float2* __restrict__ twiddle,
                                                                  const long long* __restrict__ prefix,
                                                                  unsigned long long* __restrict__ workCounter,
                                                                  int* __restrict__ done, unsigned* __restrict__ maxKey,
@@ -334,12 +335,17 @@ void launch_fused(Handle& h, const FrontendArgs& a, void* scratch)
     const size_t clear = reinterpret_cast<char*>(maxKey + a.n) - reinterpret_cast<char*>(counter);
     launch_ragged_prefix(SlotCount<S::TF>{a, a.n, a.lookahead}, nslots, prefix, h.stream(),
                          reinterpret_cast<unsigned*>(counter), int(clear / 4));
-    int grid = persistent_grid(h, reinterpret_cast<const void*>(frontend_kernel<NFFT, TFX>), kFusedThreads, lay.total);
+    // 128 points: four CTAs at 64 registers, against three at 80 without spills in the mel sweep (64 clips of 10 s, 23, 80
+    // and 128 filters 106, 122 and 142 against 122, 136 and 153 us; 256 and 512 filters, mostly sweep, 246 and 507 against 238 and 466)
+    constexpr int kCtas = NFFT <= 512 ? 3 : 2;
+    auto kernel = NFFT == 128 && a.mel.numFilter <= 200 ? frontend_kernel<NFFT, TFX, NFFT == 128 ? 4 : kCtas>
+                                                        : frontend_kernel<NFFT, TFX, kCtas>;
+    int grid = persistent_grid(h, reinterpret_cast<const void*>(kernel), kFusedThreads, lay.total);
     if (a.ctasPerSm > 0) grid = std::min(grid, a.ctasPerSm * h.num_sms());
     if (a.reserveSms > 0 && a.reserveSms < h.num_sms())
         grid = std::max(1, grid / h.num_sms() * (h.num_sms() - a.reserveSms));
     // starts while the prefix kernel runs: the tables are built before grid_dependency_wait()
-    launch_dependent(frontend_kernel<NFFT, TFX>, dim3(grid), dim3(kFusedThreads), lay.total, h.stream(),
+    launch_dependent(kernel, dim3(grid), dim3(kFusedThreads), lay.total, h.stream(),
                      "frontend_kernel", a, tw, static_cast<const long long*>(prefix), counter, done, maxKey,
                      h.device_flags(), static_cast<const uint4*>(melTables));
     count_launch();

@@ -27,7 +27,8 @@ SUITES = ["tests/test_gpu_ops.py", "tests/test_gpu_normalize_nd.py", "tests/test
           "tests/test_gpu_frontend_tc.py", "tests/test_gpu_tc.py", "tests/test_gpu_parity_reference.py",
           "tests/test_gpu_edges.py", "tests/test_gpu_parity_fuzz.py", "tests/test_gpu_nsr_intervals.py",
           "tests/test_gpu_resample_held.py", "tests/test_gpu_spectrogram_tiles.py", "tests/test_gpu_ragged_batches.py",
-          "tests/test_gpu_normalize_rows.py", "tests/test_gpu_checked_hooks.py", "tests/test_gpu_checked_fuzz.py"]
+          "tests/test_gpu_normalize_rows.py", "tests/test_gpu_frontend_128.py",
+          "tests/test_gpu_checked_hooks.py", "tests/test_gpu_checked_fuzz.py"]
 TIMED = "spread_over_the_gpu or keep_their_time"
 
 
