@@ -20,7 +20,7 @@
 // reductions, one warp per parameter for long ones (the parameter's elements staged once in shared
 // memory when contiguous; the 32 lanes take the 32 subtrees five levels down the same halving tree
 // and combine them pairwise in tree order); normalize_kernel -- one destination row per CTA step,
-// four columns per thread.  HBM-bound.
+// four columns per thread.  The first is bound by latency and instructions, the last by HBM.
 #include "common.cuh"
 #include "ops.hpp"
 

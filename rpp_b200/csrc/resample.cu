@@ -287,6 +287,23 @@ __device__ __forceinline__ void channel_taps(const W& win, const float* in, floa
         if (c < C) *RPPB_WR(out + c) = acc[c];
 }
 
+// The reference's phase sum of a block.
+__device__ __forceinline__ void block_phases(float p, float fscale, float* to)
+{
+    float4* out = reinterpret_cast<float4*>(to);
+#pragma unroll 8
+    for (int k = 0; k < kBlock / 4; ++k)
+    {
+        float4 q;
+        q.x = p;
+        q.y = p = __fadd_rn(p, fscale);
+        q.z = p = __fadd_rn(p, fscale);
+        q.w = p = __fadd_rn(p, fscale);
+        p = __fadd_rn(p, fscale);
+        out[k] = q;
+    }
+}
+
 // A unit of the flat work list, decoded by the phase warp for the compute warps.
 constexpr int kUnitSkip = 0, kUnitCopy = 1, kUnitResample = 2;
 struct UnitInfo
@@ -383,19 +400,7 @@ __global__ void __launch_bounds__(kThreads, 4)
                 const float fscale = __double2float_rn(scale);
                 const double inBlockRaw = __dmul_rn(double(u.unit * kBlock), scale);
                 u.inBlockRounded = int(inBlockRaw);
-                float p = __double2float_rn(__dsub_rn(inBlockRaw, double(int(inBlockRaw))));
-                float4* out = reinterpret_cast<float4*>(s_phase[slot][j]);
-#pragma unroll 8
-                for (int k = 0; k < kBlock / 4; ++k)
-                {
-                    float4 q;
-                    q.x = p;
-                    q.y = p = __fadd_rn(p, fscale);
-                    q.z = p = __fadd_rn(p, fscale);
-                    q.w = p = __fadd_rn(p, fscale);
-                    p = __fadd_rn(p, fscale);
-                    out[k] = q;
-                }
+                block_phases(__double2float_rn(__dsub_rn(inBlockRaw, double(int(inBlockRaw)))), fscale, s_phase[slot][j]);
                 // ask L2 for the unit's input span (a group ahead of its use): the taps of its outputs
                 // read samples [ceil(first phase) - lobes, ceil(last phase) + lobes) from inBlockRounded on
                 const int cnt = min(kBlock, u.outEnd - u.unit * kBlock);
@@ -684,23 +689,6 @@ struct HeldItem
     int kind[kItemBlocks];
     float first[kItemBlocks];  // its first phase
 };
-
-// The reference's phase sum of a block.
-__device__ __forceinline__ void block_phases(float p, float fscale, float* to)
-{
-    float4* out = reinterpret_cast<float4*>(to);
-#pragma unroll 8
-    for (int k = 0; k < kBlock / 4; ++k)
-    {
-        float4 q;
-        q.x = p;
-        q.y = p = __fadd_rn(p, fscale);
-        q.z = p = __fadd_rn(p, fscale);
-        q.w = p = __fadd_rn(p, fscale);
-        p = __fadd_rn(p, fscale);
-        out[k] = q;
-    }
-}
 
 // The item's blocks that do not share its weights, an output per thread with the reference's operations.  Not
 // inlined: its registers would come on top of the held weights.

@@ -38,6 +38,13 @@ struct Plan<1024> { static constexpr int R1 = 32, R2 = 16, TF = 16; };
 template <>
 struct Plan<2048> { static constexpr int R1 = 32, R2 = 32, TF = 16; };
 
+// The sizes whose packed transform is R x R points: stft_pair.cuh's tile.
+template <int NFFT>
+struct PairPlan
+{
+    static constexpr bool use = NFFT == 128 || NFFT == 512;
+};
+
 // TFX: frames per tile (Plan<NFFT>::TF by default; the fused kernel also instantiates other sizes,
 // which change the schedule and never the arithmetic of a frame).
 template <int NFFT, int THREADS, int TFX = Plan<NFFT>::TF>
@@ -66,7 +73,7 @@ struct StftShape
     // reads a full nfft-sample buffer without bounds checks (the window is 0 outside [0, W)).
     __host__ __device__ static int span_pad(int W)
     {
-        return (window_offset(W) + (NFFT == 128 || NFFT == 512 ? 4 : 3)) & ~3;
+        return (window_offset(W) + (PairPlan<NFFT>::use ? 4 : 3)) & ~3;
     }
     __host__ __device__ static int span_tail(int W)
     {

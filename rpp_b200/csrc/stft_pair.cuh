@@ -6,7 +6,7 @@
 //   - the bins k and M - k that the unpack pairs lie in lanes j and R - j of the frame's lanes, so they meet by warp
 //     shuffles and the transform is not stored again;
 //   - the power of frames f and f + 1, which one warp transforms, replaces their exchange slots, so a 16-frame
-//     tile needs 33 KB instead of 53 KB and four CTAs of 256 threads fit an SM (at 64 registers), not three;
+//     tile needs 35 KB instead of 53 KB and four CTAs of 256 threads fit an SM (at 64 registers), not three;
 //   - the window is halved (exact), which takes the place of the unpack's factors of 1/2;
 //   - the next tile's samples are copied into the span buffer while this tile is transformed.
 // On 256 clips of 1 to 16 s (nfft 512) the spectrogram kernel takes 176 us instead of 221 (ncu) and the fused front
@@ -19,12 +19,6 @@
 #include "stft.cuh"
 
 namespace rppb {
-
-template <int NFFT>
-struct PairPlan
-{
-    static constexpr bool use = NFFT == 128 || NFFT == 512;
-};
 
 template <int NFFT>
 struct PairShape
