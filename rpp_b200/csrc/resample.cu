@@ -1044,13 +1044,15 @@ void launch_resample(Handle& h, void* scratch, const float* src, uint32_t srcStr
     const bool magic = resample_magic_ok(w, pairs);
     const bool fma = resample_scale_pow2(w);
     resample_exact_range(w, magic, fma);
-    // The held-weights kernel pays from two full items per CTA on, 9472 blocks at 2 CTAs per SM, 2.5 minutes at 16 kHz
-    // (against resample_kernel, mono / stereo from 44.1 kHz: 8 clips of 10 s 42 and 48, 56 and 54 us; 16 clips 56 and
-    // 81, 69 and 95 us; from 48 kHz 41 and 34, 48 and 48; 50 and 56, 68 and 83 us).  resample_split_kernel counts them;
-    // it and the second kernel cost 2 us, so batches that are below twice that when padded skip both.
+    // The held-weights kernel pays from one full item per CTA on, 4736 blocks at 2 CTAs per SM, 1.3 minutes at 16 kHz, and
+    // from one and a half when it down-mixes (against resample_kernel, clips of mixed rates: mono 4236 blocks 34 and 35
+    // us, 4926 35 and 39, 6895 41 and 50, 9064 44 and 62; stereo 4926 50 and 44 us, 6416 56 and 56, 7135 54 and 58, 9311
+    // 67 and 76).  resample_split_kernel counts them; it and the second kernel cost 2 to 4 us, so batches that are below
+    // four items per CTA when padded skip both.
     const long long padded = (long long)n * ((dstStride + kBlock - 1) / kBlock);
-    const int minBlocks = 2 * kItemBlocks * kHeldCtas * h.num_sms();
-    const bool split = padded >= 2ll * minBlocks && (downmix || channels <= 1) && resample_held_ok(w, magic, fma);
+    const int items = kItemBlocks * kHeldCtas * h.num_sms();
+    const int minBlocks = downmix ? items + items / 2 : items;
+    const bool split = padded >= 4ll * items && (downmix || channels <= 1) && resample_held_ok(w, magic, fma);
     if (split)
     {
         auto held = downmix ? launch_held<true> : launch_held<false>;
