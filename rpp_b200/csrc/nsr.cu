@@ -19,13 +19,13 @@
 //   1. energy_kernel: FP64 energies of 64-sample chunks, one streaming pass over the signal (HBM-bound: 30 us
 //      for 256 clips of 1 to 16 s, 4.6 TB/s);
 //   2. region_kernel: one CTA per sample: scan of the energies, cutoff interval, both ends, replays (15 to
-//      20 us without a replay, about 50 us more for each one);
-//   3. exact_kernel: the reset blocks of the samples that are left, over the whole GPU (3 us with none).
+//      20 us without a replay, about 45 us more for each one);
+//   3. exact_kernel: the reset blocks of the samples that are left, over the whole GPU (2 us with none).
 // A clip that ends in silence after sound within one reset block needs a replay as a rule: its running
 // sum decays to rounding residue, which no bound can place against the cutoff.  The bare chain is
 // latency-bound (8 cycles per sample, 38 us for a block of 8192 with a window of 2048).
-// Replaying every block of every clip and searching the stored values, as an earlier version did, took 288 us per call
-// on this batch; now 52 us where no clip needs a replay, 104 to 171 us (over the signals) where most do.
+// Replaying every block of every clip and searching the stored values, as an earlier version did, took 271 to 303 us per
+// call on this batch; now 52 us where no clip needs a replay, 92 to 147 us, over eight signals, where most do.
 // Where every block is replayed (the rule in launch_nsr and region_kernel's `full`) the call costs, against that
 // version: the same batch with a window of 200 193 for 376 us, 512 clips of 10 s with a window of 16 267 for 497 us, 10
 // minutes in one clip with a window of 200 116 for 167 us and without resets 101 for 113 ms; the blocks replayed by
@@ -55,7 +55,7 @@ struct ReplayShape
 using OneShape = ReplayShape<kThreads / 32 - 1, 256>;    // region_kernel: one block, seldom a few
 using ManyShape = ReplayShape<28, 128>;                  // exact_kernel: two CTAs per SM
 constexpr int kRun = 1024, kRuns = 512;        // largest_window: samples per run, runs whose maxima are kept
-constexpr int kSearch = 512;                   // chunks that largest_window searches at most (30 us)
+constexpr int kSearch = 1024;                  // chunks that largest_window searches at most (50 us; giving up costs 100)
 constexpr double kLongChain = 49152.0;         // operations of a reset block's chain from which region_kernel replays none
 constexpr int kTallyShift = 36;                // ExactList::tally: clips above, reset blocks (2^36: 256 GB of floats) below
 constexpr int kMaxClips = 1 << 27;             // per launch
@@ -635,7 +635,7 @@ __device__ __forceinline__ void write_region(int first, int last, int W, int b, 
 __global__ void __launch_bounds__(kThreads) region_kernel(const float* __restrict__ src, uint32_t stride,
                                                           const int* __restrict__ len, int windowLength, int reset,
                                                           float referencePower, float cutOff, double* __restrict__ energies,
-                                                          long long pitch, bool intervals, ExactList exact,
+                                                          long long pitch, bool intervals, bool local, ExactList exact,
                                                           int* __restrict__ outBegin, int* __restrict__ outLength)
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -650,7 +650,8 @@ __global__ void __launch_bounds__(kThreads) region_kernel(const float* __restric
         if (tid == 0) write_region(-1, -1, windowLength, b, outBegin, outLength);
         return;
     }
-    // leaves the clip to exact_kernel
+    // leaves the clip to exact_kernel (never with `local`: then its blocks fit a replay here, and that kernel is not
+    // launched)
     auto pass_on = [&](int blocks) {
         const unsigned long long t =
             atomicAdd(RPPB_WR(dependency_result(exact.tally)), 1ull << kTallyShift | (unsigned long long)blocks);
@@ -843,6 +844,36 @@ __global__ void __launch_bounds__(kThreads) region_kernel(const float* __restric
             full = first < kNone || last < kNone;
         }
     }
+    if (full && local)
+    {
+        clip.P = clip.all;
+        auto all = [&](float cut) {
+            __syncthreads();
+            if (tid < blocks)
+            {
+                sh.set(tid, clip.x, L, clip.W, tid * clip.R, clip.R);
+                sh.low[tid] = sh.high[tid] = cut;
+            }
+            __syncthreads();
+            replay<OneShape, true>(sh, buf, blocks, clip.W, clip.meanFactor);
+        };
+        float base = referencePower;
+        if (peakRef)
+        {
+            all(INFINITY);
+            base = -FLT_MAX;
+            for (int j = 0; j < blocks; ++j) base = fmaxf(base, sh.peak[j]);
+        }
+        all(__fmul_rn(base, cutOff));
+        first = last = -1;
+        for (int j = 0; j < blocks; ++j)
+        {
+            if (sh.lastLow[j] < 0) continue;
+            if (first < 0) first = sh.firstLow[j];
+            last = sh.lastLow[j];
+        }
+        full = false;
+    }
     if (tid != 0) return;
     if (full) pass_on(blocks);
     else write_region(first, last, windowLength, b, outBegin, outLength);
@@ -1027,6 +1058,9 @@ void launch_nsr(Handle& h, void* scratch, const NsrArgs& a)
     list.blockMax = cv.take<float>(block_count(a.n, a.srcStride, a.resetInterval));
     // the intervals' chunks have to resolve the window and the reset blocks; else exact_kernel takes every clip
     const bool intervals = a.windowLength >= 4 * kSub && (a.resetInterval == -1 || a.resetInterval >= kSub);
+    // samples of few reset blocks are finished by region_kernel whatever their intervals say, and a launch is saved (one
+    // clip of 1 s 16.0 -> 12.4 us)
+    const bool local = intervals && block_count(1, a.srcStride, a.resetInterval) <= OneShape::kChains;
     const int ups = int(a.srcStride / kUnit) + 1;
     for (int b0 = 0; b0 < a.n; b0 += kMaxClips)
     {
@@ -1042,8 +1076,9 @@ void launch_nsr(Handle& h, void* scratch, const NsrArgs& a)
         persistent_grid(h, reinterpret_cast<const void*>(region_kernel), kThreads, OneShape::kBytes);   // shared-memory opt-in
         launch_dependent(region_kernel, dim3(n), dim3(kThreads), OneShape::kBytes, h.stream(), "region_kernel", src,
                          a.srcStride, a.len + b0, a.windowLength, a.resetInterval, a.referencePower, a.cutOff, energies,
-                         pitch, intervals, list, a.begin + b0, a.length + b0);
+                         pitch, intervals, local, list, a.begin + b0, a.length + b0);
         count_launch();
+        if (local) continue;
         const int exactGrid = persistent_grid(h, reinterpret_cast<const void*>(exact_kernel), kThreads, ManyShape::kBytes);
         launch_dependent(exact_kernel, dim3(exactGrid), dim3(kThreads), ManyShape::kBytes, h.stream(), "exact_kernel", src,
                          a.srcStride, a.len + b0, a.windowLength, a.resetInterval, a.referencePower, a.cutOff, list,
