@@ -336,7 +336,8 @@ void launch_fused(Handle& h, const FrontendArgs& a, void* scratch)
     launch_ragged_prefix(SlotCount<S::TF>{a, a.n, a.lookahead}, nslots, prefix, h.stream(),
                          reinterpret_cast<unsigned*>(counter), int(clear / 4));
     // 128 points: four CTAs at 64 registers, against three at 80 without spills in the mel sweep (64 clips of 10 s, 23, 80
-    // and 128 filters 106, 122 and 142 against 122, 136 and 153 us; 256 and 512 filters, mostly sweep, 246 and 507 against 238 and 466)
+    // and 128 filters 106, 122 and 142 against 122, 136 and 153 us; 256 and 512 filters, mostly sweep, 246 and 507
+    // against 238 and 466)
     constexpr int kCtas = NFFT <= 512 ? 3 : 2;
     auto kernel = NFFT == 128 && a.mel.numFilter <= 200 ? frontend_kernel<NFFT, TFX, NFFT == 128 ? 4 : kCtas>
                                                         : frontend_kernel<NFFT, TFX, kCtas>;

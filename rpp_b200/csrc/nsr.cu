@@ -15,7 +15,8 @@
 // replayed, in exactly the reference's order (add the new square, store sum * (1/windowLength), subtract
 // the square leaving the window; explicit round-to-nearest intrinsics, no FMA), and, if its exact values
 // lie inside the cutoff's interval too, the blocks that may hold the maximum.  Clips that this does not settle have
-// every block replayed, and many short ones have from the start (nsr_stored.cu).  Begin and length are therefore the host path's on every input.
+// every block replayed, and many short ones have from the start (nsr_stored.cu).  Begin and length are
+// therefore the host path's on every input.
 //   1. energy_kernel: FP64 energies of 64-sample chunks, one streaming pass over the signal (HBM-bound: 30 us
 //      for 256 clips of 1 to 16 s, 4.6 TB/s);
 //   2. region_kernel: one CTA per sample: scan of the energies, cutoff interval, both ends, replays (15 to

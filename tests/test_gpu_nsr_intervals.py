@@ -107,6 +107,27 @@ def test_many_clips_with_every_block_replayed(gpu, oracle, reset, window, ref):
     np.testing.assert_array_equal(length, l_ref)
 
 
+@pytest.mark.parametrize("scale", [1.0, 1e-18])   # 1e-18: intervals do not hold, every block is replayed
+@pytest.mark.parametrize("cut", [-60.0, -0.01, 0.0])
+@pytest.mark.parametrize("blocks", [7, 8])
+def test_few_blocks(gpu, oracle, blocks, cut, scale):
+    """As many reset blocks as the CTA of a clip replays itself, and one more."""
+    r = np.random.default_rng(16)
+    n, reset, window = 40, 700, 300
+    width = blocks * reset
+    lens = r.integers(width - 2 * reset, width + 1, n).astype(np.int32)
+    lens[:2] = width, width - reset
+    x = np.zeros((n, width), np.float32)
+    for i, k in enumerate(lens):
+        v = r.normal(0, 0.2, k) if i % 3 else 0.2 * np.sin(np.arange(k) * 0.03)
+        v[k - 90 * (i % 5):] = 0.0
+        x[i, :k] = v * scale
+    b_ref, l_ref = oracle.nsr(x, lens, cut, window, 0.0, reset)
+    begin, length, _ = detect(gpu, x, lens, window, reset, cut)
+    np.testing.assert_array_equal(begin, b_ref)
+    np.testing.assert_array_equal(length, l_ref)
+
+
 @pytest.mark.parametrize("reset,window,top", [(8192, 2048, 9000), (8192, 512, 1500), (512, 300, 3000),
                                                (-1, 2048, 9000), (8192, 100, 2000), (30, 40, 900), (8192, 9000, 3000)])
 @pytest.mark.parametrize("n", [1023, 1024, 1500])
