@@ -49,8 +49,10 @@ def setup(rates, channels, seed, reps, outs=OUTS):
 
 
 def call(gpu, s, out, width):
-    lut, scale, center, lobes = kaiser_sinc(16)
-    s.setdefault("lut", dev(lut))
+    if "lut" not in s:
+        lut, *s["table"] = kaiser_sinc(16)
+        s["lut"] = dev(lut)
+    scale, center, lobes = s["table"]
     ch = s["channels"]
     sd, od = audio_desc(s["n"], s["L"], channels=ch, num_dims=3 if ch > 1 else 2), audio_desc(s["n"], width)
     if ch > 1:
@@ -109,24 +111,24 @@ def test_mixed_batch_equals_oracle(gpu, oracle, rates):
     assert bool((out.view(reps, n, width).view(torch.int32) == dev(ref).view(torch.int32)).all())
 
 
-@pytest.mark.parametrize("rates,channels", [((48000, 44100), 1), ((16000, 44100), 2), ((96000, 16000), 2)])
-def test_rates_that_share_no_weights_keep_their_time(gpu, rates, channels):
-    """One large batch against its four quarters, which are too small for the held-weights kernel: with that kernel on
-    such rates the batch takes 2.5 times its quarters or more."""
-    s, _, _ = setup(rates, channels, 3, 24, outs=[110000, 109000])
-    q = dict(s, n=s["n"] // 4, x=s["x"][:s["n"] // 4], dims=s["dims"][:s["n"] // 4])
-    assert s["n"] * -(-s["width"] // 256) >= padded_blocks_needed() > q["n"] * -(-s["width"] // 256)
-
-    def best(v):
-        out = canvas((v["n"], v["width"]))
+@pytest.mark.parametrize("rates,channels,bound", [((48000, 44100), 1, 3.0), ((16000, 44100), 1, 3.0),
+                                                  ((96000, 16000), 2, 6.0)])
+def test_rates_that_share_no_weights_keep_their_time(gpu, rates, channels, bound):
+    """Against as many outputs at a rate that shares weights (44.1 to 48 kHz): 1.7, 1.6 and 2.6 times the time; with the
+    held-weights kernel on such rates, where it gains nothing, 5, 5 and 10 times."""
+    def best(rates):
+        s, _, _ = setup(rates, channels, 3, 40, outs=[110000, 109000])
+        assert s["n"] * -(-s["width"] // 256) >= padded_blocks_needed()
+        out = canvas((s["n"], s["width"]))
         times = []
         for _ in range(8):
             a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             a.record()
-            assert call(gpu, v, out, v["width"]) == 0
+            for _ in range(10):
+                assert call(gpu, s, out, s["width"]) == 0
             b.record()
             b.synchronize()
             times.append(a.elapsed_time(b))
         return min(times)
 
-    assert best(s) < 1.5 * 4 * best(q)
+    assert best(rates) < bound * best((44100, 48000))
